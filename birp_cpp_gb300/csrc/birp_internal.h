@@ -186,7 +186,7 @@ cudaError_t launch_render_plain(const RequestDev& req, KernelStats* stats, cudaS
 // (fewer registers, more resident warps than the general kernel), the same in
 // the compact and in the pairs layout, CMEM requests, nearest-mode cube
 // requests (any layout), trilinear requests of cubes holding a negative value
-// (any layout; FP64 sums next to negative nodes), and the general kernel that
+// (any layout; float-float sums and signs next to negative nodes), and the general kernel that
 // renders any request (used where one launch must take a mix, see
 // birp_batch_render_noalloc).
 enum BatchClass : int {

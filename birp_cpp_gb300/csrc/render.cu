@@ -53,7 +53,9 @@ constexpr int kThreads = 128;
 #define BIRP_CMEM_MINB BIRP_CMEM_MINB_TUNED  // CMEM
 #endif
 #ifndef BIRP_SIGNED_MINB
-#define BIRP_SIGNED_MINB 4  // trilinear cubes holding negative values (any layout, FP64 cell sums)
+// trilinear cubes holding negative values (any layout; at 5 or 6 CTAs per SM
+// the float-float cell function spills: 12 orbit renders 2.21 -> 4.13 / 5.12 ms)
+#define BIRP_SIGNED_MINB 4
 #endif
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
@@ -636,11 +638,6 @@ __device__ __forceinline__ double node_value(const CubeDev& C, int i, int j, int
 #endif
 }
 
-// Whether in-box sample i of a ray is below zero in the FP64 oracle's own
-// arithmetic (cube64_sample at pos64, direction rebuilt from the tile's
-// column/row terms a + b): the exact cell of each coordinate (g: the FP32
-// guesses), FP64 fractions and lerps x -> y -> z, or the lower node's value
-// for nearest. Not inlined: it runs only for samples in flagged cells.
 // The FP64 oracle's value of in-box sample i of a ray (cube64_sample at
 // pos64 = P + d ((i + 1/2) dt), d the ray's FP64 direction): the exact cell of
 // each coordinate (g: guesses, updated to the cells found), FP64 fractions and
@@ -665,82 +662,162 @@ __device__ __forceinline__ double sample_value64(const CubeDev& C, int trilinear
   return lerp64(lerp64(lx1, lx2, f[1]), lerp64(hx1, hx2, f[1]), f[2]);
 }
 
-__device__ __noinline__ bool sample_negative64(const CubeDev* Cp, int trilinear, const double* a, const double* b,
-                                               double px, double py, double pz, double dt, int i, int g0, int g1,
-                                               int g2) {
+// The same with the ray's FP64 direction rebuilt from the tile's column and
+// row terms (a, b). Not inlined: it runs only where float-float cannot decide.
+__device__ __noinline__ double ray_value64(const RequestDev* Rp, const double* a, const double* b, int i, int g0,
+                                           int g1, int g2) {
   double w[3], d[3];
   for (int r = 0; r < 3; ++r) w[r] = __dadd_rn(a[r], b[r]);
   dir64(w, d);
-  const double P[3] = {px, py, pz};
   int g[3] = {g0, g1, g2};
-  return sample_value64(*Cp, trilinear, d, P, dt, i, g) < 0.0;
+  return sample_value64(*Rp->cube, 1, d, Rp->pos, Rp->dt, i, g);
 }
 
-// Sum, in FP64, of the FP64 oracle's values of the trilinear samples
-// [i0, i1) of a ray (its FP64 direction rebuilt from the tile terms a + b; g:
-// the cell of the walk, a guess of the exact cells). The trilinear march of a
-// cube holding negative values takes it for a cell next to a negative node:
-// there corners of both signs cancel, and an FP32 interpolation keeps only
-// ~1e-7 of the corners' size, while a run that ends at a zero crossing may
-// be short. Not inlined: it runs only in such cells.
-__device__ __noinline__ double samples_sum64(const CubeDev* Cp, const double* a, const double* b, double px,
-                                             double py, double pz, double dt, int i0, int i1, int g0, int g1,
-                                             int g2) {
-  double w[3], d[3];
-  for (int r = 0; r < 3; ++r) w[r] = __dadd_rn(a[r], b[r]);
-  dir64(w, d);
-  const double P[3] = {px, py, pz};
-  int g[3] = {g0, g1, g2};
-  double s = 0.0;
-  for (int i = i0; i < i1; ++i) s = __dadd_rn(s, sample_value64(*Cp, 1, d, P, dt, i, g));
-  return s;
-}
+// A ray over a cube holding negative values ends at its first negative sample
+// (PREFIX), or skips negative samples to the first good one and ends at the
+// next (CLIP); each lane walks its own contiguous part of the ray. What a
+// lane reports, in the order the samples lie: the sum of its first block of
+// good samples, whether it has one, whether a negative sample ended it, and
+// whether its first sample is negative.
+enum RunPhase : int { RUN_SKIP = 0, RUN_GOOD = 1, RUN_ENDED = 2 };
+struct LaneRun {
+  int phase;       // RUN_SKIP: no good sample yet (CLIP), RUN_GOOD: in the block, RUN_ENDED: past it
+  bool first_neg;  // the lane's first sample is negative
+  int n;           // samples of the block
+};
 
-// First sample in [lo, hi) of this lane's ray that is below zero (want_neg)
-// or not (!want_neg); hi if none. The ray's S lanes test S consecutive
-// samples per step and stop together at the first hit. A sample is tested in
-// FP64 only when its FP32 cell is flagged (the flags cover one cell around
-// every negative corner, and the FP32 cell is within one of the exact cell
-// unless all_exact, which tests every sample). Every lane of the warp calls.
-// (d0..d2: the ray's FP32 direction; a / b: the tile terms of its FP64
-// direction.) Inlined: a call costs the walks more in saved registers.
-__device__ __forceinline__ int neg_search(const RequestDev* Rp, float d0, float d1, float d2, const double* a,
-                                       const double* b, int S, int seg, int lo, int hi, bool want_neg,
-                                       bool all_exact) {
+// The trilinear samples [i0, i1) of a ray in a cell next to a negative node
+// (flag set): the run's state goes on from sample to sample, and the good
+// samples' values are summed into *sum. There corners of both signs may
+// cancel, an FP32 interpolation keeps only ~1e-7 of the corners' size and a
+// run that ends at a zero crossing may be short, so position, cell, fractions
+// and interpolation are float-float (~46 bits, on the FP32 pipes: FP64 is 1/58
+// of their rate). A sample's cell and sign are decided within the stated
+// bounds of that arithmetic, which cover the oracle's own FP64 rounding; what
+// they leave open (and corners that are not finite) takes the oracle's FP64.
+// Bound by the rays that enter such cells (latency: 16 warps per SM, the
+// function's registers). 12 orbit renders of a 192x160x176 cube with 1e-5 of
+// its nodes negative: 16.5 ms with a scan of every sample before the walk and
+// FP64 signs and sums, 2.21 ms so.
+// (g0..g2: the walk's cell, a guess.) Not inlined: it runs only in such cells.
+__device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* a, const double* b, int i0, int i1,
+                                            int g0, int g1, int g2, LaneRun run, int first, float2* sum) {
   const RequestDev& R = *Rp;
   const CubeDev& C = *R.cube;
-  const float st[3] = {R.dt32 * d0, R.dt32 * d1, R.dt32 * d2};
-  int found = hi;
-  for (int base = lo; __any_sync(0xffffffffu, base < found); base += S) {
-    const int i = base + seg;
-    bool hit = false;
-    if (base < found && i < hi) {
-      int g[3];
+  FF wf[3], st[3], bs[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const AxisDev& A = C.ax[k];
-        const float x = fmaf((float)i + 0.5f, st[k], R.pos32[k]);
-        const float idx = A.uniform ? (x - A.c0) * A.inv_h : lut_index(A, C.lut, x);
-        int kb;
-        magic_floor(fminf(fmaxf(idx, 0.f), (float)(A.n - 2)), kb);
-        g[k] = kb - kMagicBits;
-      }
-      bool neg = false;
-#ifdef BIRP_DEBUG_BOUNDS
-      long long fi = ((long long)g[2] * C.ax[1].n + g[1]) * C.ax[0].n + g[0];
-      if (!bound_ok(fi, C.neg_n, 3)) fi = 0;
-      if (all_exact || __ldg(C.negflag + fi))
-#else
-      if (all_exact || __ldg(C.negflag + ((size_t)g[2] * C.ax[1].n + g[1]) * C.ax[0].n + g[0]))
-#endif
-        neg = sample_negative64(R.cube, R.interp, a, b, R.pos[0], R.pos[1], R.pos[2], R.dt, i, g[0], g[1], g[2]);
-      hit = neg == want_neg;
-    }
-    int cand = hit ? i : hi;
-    for (int o = S >> 1; o >= 1; o >>= 1) cand = min(cand, __shfl_xor_sync(0xffffffffu, cand, o));
-    found = min(found, cand);
+  for (int r = 0; r < 3; ++r) {
+    const double w = __dadd_rn(a[r], b[r]);
+    const float h = (float)w;
+    wf[r] = {h, (float)(w - (double)h)};
   }
-  return found;
+  const FF rs = ff_rsqrt(ff_add(ff_add(ff_mul(wf[0], wf[0]), ff_mul(wf[1], wf[1])), ff_mul(wf[2], wf[2])));
+  // bound on |float-float position - the oracle's FP64 position| per axis
+  float e[3];
+  int k[3] = {g0, g1, g2};
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const AxisDev& A = C.ax[r];
+    st[r] = ff_mul(ff_mul(wf[r], rs), {R.dt_hi, R.dt_lo});
+    bs[r] = ff_add({R.pos_hi[r], R.pos_lo[r]}, {0.5f * st[r].hi, 0.5f * st[r].lo});
+    e[r] = 2e-13f * (fabsf(R.pos32[r]) + (float)R.N * R.dt32 + fmaxf(fabsf((float)A.c_first), fabsf((float)A.c_last)));
+    k[r] = min(max(k[r], 0), A.n - 2);
+  }
+  FF s = {sum->x, sum->y};
+  for (int i = i0; i < i1 && run.phase != RUN_ENDED; ++i) {
+    FF f[3];
+    float e_rel = 0.f;  // sum of e / cell width
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const AxisDev& A = C.ax[r];
+      const FF x = ff_add(bs[r], ff_mul(st[r], {(float)i, 0.f}));
+      // whether the oracle's position lies below node j
+      auto below = [&](int j) {
+        const float2 c = __ldg(C.nodes_ff[r] + j);
+        const float diff = (x.hi - c.x) + (x.lo - c.y);
+        if (fabsf(diff) > e[r]) return diff < 0.f;
+        double w[3], d[3];
+        for (int q = 0; q < 3; ++q) w[q] = __dadd_rn(a[q], b[q]);
+        dir64(w, d);
+        return pos64(R.pos[r], d[r], R.dt, i) < A.c64[j];
+      };
+      while (k[r] > 0 && below(k[r])) --k[r];
+      while (k[r] < A.n - 2 && !below(k[r] + 1)) ++k[r];
+      const float2 c0 = __ldg(C.nodes_ff[r] + k[r]), c1 = __ldg(C.nodes_ff[r] + k[r] + 1);
+      const FF iw = ff_recip(ff_add({c1.x, c1.y}, {-c0.x, -c0.y}));
+      f[r] = ff_mul(ff_add(x, {-c0.x, -c0.y}), iw);
+      e_rel = fmaf(e[r], iw.hi, e_rel);
+    }
+    float v[8], mn = INFINITY, mx = -INFINITY, size = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      v[q] = node_value(C, k[0] + (q & 1), k[1] + ((q >> 1) & 1), k[2] + (q >> 2));
+      mn = fminf(mn, v[q]);
+      mx = fmaxf(mx, v[q]);
+      size += fabsf(v[q]);
+    }
+    bool neg;
+    FF val = {0.f, 0.f};
+    bool open = !(size < 1e37f);  // NaN, infinite or near-overflow corners
+    if (!open) {
+      if (mx < 0.f) {
+        neg = true;  // every interpolation of negative corners is
+      } else {
+        auto lerp = [](FF p, FF q, FF t) { return ff_add(p, ff_mul(ff_add(q, {-p.hi, -p.lo}), t)); };
+        auto lerp1 = [](float p, float q, FF t) {
+          float d, r;
+          two_sum(q, -p, d, r);
+          return ff_add({p, 0.f}, ff_mul({d, r}, t));
+        };
+        val = lerp(lerp(lerp1(v[0], v[1], f[0]), lerp1(v[2], v[3], f[0]), f[1]),
+                   lerp(lerp1(v[4], v[5], f[0]), lerp1(v[6], v[7], f[0]), f[1]), f[2]);
+        neg = val.hi < 0.f;
+        // with every corner >= 0 the oracle's interpolation is not negative;
+        // else the sign is certain beyond the error of the value
+        if (mn >= 0.f) neg = false;
+        else open = !(fabsf(val.hi) > size * fmaf(4.f, e_rel, 4e-12f));
+      }
+    }
+    if (open) {
+      const double d = ray_value64(Rp, a, b, i, k[0], k[1], k[2]);
+      neg = d < 0.0;
+      const float h = (float)d;
+      val = {h, isfinite(h) ? (float)(d - (double)h) : 0.f};
+    }
+    if (i == first) run.first_neg = neg;
+    if (neg) {
+      if (run.phase == RUN_GOOD) run.phase = RUN_ENDED;
+    } else {
+      run.phase = RUN_GOOD;
+      ++run.n;
+      s = isfinite(val.hi) ? ff_add(s, val) : FF{s.hi + val.hi, 0.f};
+    }
+  }
+  *sum = make_float2(s.hi, s.lo);
+  return run;
+}
+
+// Whether this lane's block of good samples is part of its ray's run, from
+// the reports of the ray's S lanes in sample order: the run begins with the
+// first in-box sample (PREFIX) or the first good one (CLIP) and ends at the
+// next negative sample, in whichever lane it lies. Every lane of the warp
+// calls; `count`: the lane's samples.
+__device__ __forceinline__ bool lane_in_run(const LaneRun& run, int count, int mode, int S, int seg, int lane) {
+  const int code = (count > 0 ? 1 : 0) | (run.n > 0 ? 2 : 0) | (run.phase == RUN_ENDED ? 4 : 0) | (run.first_neg ? 8 : 0);
+  int state = mode == MARCH_PREFIX ? RUN_GOOD : RUN_SKIP;
+  bool mine = false;
+  for (int j = 0; j < S; ++j) {
+    const int c = __shfl_sync(0xffffffffu, code, (lane & ~(S - 1)) + j);
+    if (!(c & 1) || state == RUN_ENDED) continue;
+    if (state == RUN_GOOD && (c & 8)) {
+      state = RUN_ENDED;
+      continue;
+    }
+    if (seg == j) mine = true;
+    if (c & 4) state = RUN_ENDED;
+    else if (c & 2) state = RUN_GOOD;
+  }
+  return mine;
 }
 
 // ---------------------------------------------------------------- one tile
@@ -759,7 +836,9 @@ enum Axes { AXES_NONE = 0, AXES_DDA = 2, AXES_DDA_COMPACT = 3, AXES_DDA_PAIRS = 
 // P: a CMEM model passed as a kernel parameter (nullptr: none); CMEM
 // requests whose model it is read its constants from the parameter space.
 // SIGNED: the trilinear march of a cube holding negative values, which sums
-// the cells next to a negative node in FP64 (samples_sum64).
+// the cells next to a negative node in float-float (signed_cell) and finds the
+// run's ends there; the nearest march of such a cube finds them by the cells'
+// own values.
 template <int KIND, int INTERP, int AXES, bool SIGNED = false>
 __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty, TileSmem& sm,
                                             KernelStats* stats, const CmemParam* P = nullptr) {
@@ -946,35 +1025,11 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     if (b < a) b = a;
   }
   if (!valid) { a = 0; b = 0; }
-  if constexpr (KIND == SPACE_CUBE) {
-    // A value below zero ends the run as the box edge does: the reference
-    // stops at its first sample < 0 (src/Camera.cpp:205-209), the -1 outside
-    // the box and negative field values alike. Cubes holding a negative value
-    // carry flags; their rays look for the first negative sample of the
-    // in-box run (PREFIX), or skip negative samples to the first good one and
-    // then look for the next negative (CLIP), before the run is summed.
-    const CubeDev& C = *R.cube;
-    if (C.negflag) {
-      // bound on |FP32 cell index - exact index|: position error (step,
-      // position and coordinate roundings) over the smallest cell, the
-      // index rounding and the uniform-axis tolerance; one cell or more and
-      // the flags' one-cell margin does not cover it
-      const float e_pos = 4e-7f * ((float)N * R.dt32 + fabsf(R.pos32[0]) + fabsf(R.pos32[1]) + fabsf(R.pos32[2]) +
-                                   C.neg_cmax) + 1e-6f;
-      const bool all_exact = fmaf(e_pos, C.neg_inv_gap, 2e-6f * (float)C.neg_nmax + 1e-6f) >= 1.f;
-      const double* ta = sm.A[lx];
-      const double* tb = sm.B[ly];
-      auto search = [&](int lo, int hi, bool want_neg) {
-        return neg_search(&R, d32[0], d32[1], d32[2], ta, tb, S, seg, lo, hi, want_neg, all_exact);
-      };
-      if (R.mode == MARCH_PREFIX) {
-        b = search(a, b, true);
-      } else {
-        a = search(a, b, false);
-        b = search(a, b, true);
-      }
-    }
-  }
+  // A value below zero ends the run as the box edge does: the reference stops
+  // at its first sample < 0 (src/Camera.cpp:205-209), the -1 outside the box
+  // and negative field values alike. SIGNED marches (cubes holding a negative
+  // value) find it as they walk.
+  [[maybe_unused]] LaneRun run{R.mode == MARCH_PREFIX ? RUN_GOOD : RUN_SKIP, false, 0};
 
   Kahan acc;
   const int first = a + seg;
@@ -1077,6 +1132,17 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
       const float ub = (float)count;
       float u = 0.f;
       float ncell = 0.f;  // cells summed: at most 2^22, exact
+      [[maybe_unused]] int cj[3] = {k0s[0], k0s[1], k0s[2]};
+      [[maybe_unused]] bool all_exact = false;
+      if constexpr (SIGNED) {
+        // bound on |FP32 cell index - exact index|: position error (step,
+        // position and coordinate roundings) over the smallest cell, the
+        // index rounding and the uniform-axis tolerance; one cell or more
+        // and the flags' one-cell margin does not cover it
+        const float e_pos = 4e-7f * ((float)N * R.dt32 + fabsf(R.pos32[0]) + fabsf(R.pos32[1]) + fabsf(R.pos32[2]) +
+                                     C.neg_cmax) + 1e-6f;
+        all_exact = fmaf(e_pos, C.neg_inv_gap, 2e-6f * (float)C.neg_nmax + 1e-6f) >= 1.f;
+      }
       while (u < ub) {
         float4 lo, hi;  // {c0, c3, c1, c5}, {c2, c6, c4, c7}
         if constexpr (COMPACT) {
@@ -1125,31 +1191,32 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         // the first sample past the cell; not behind u, where a plane passed
         // before sample u is still to be stepped (such a cell holds no sample)
         const float nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
-        // a cube holding negative values: a cell next to a negative node
-        // (its flag) is summed sample by sample in the FP64 oracle's own
-        // arithmetic; its cell per axis is the walk table position
+        // a cube holding negative values: the samples of a cell next to a
+        // negative node (its flag) are looked at one by one; an unflagged
+        // cell's are all good, as its FP32 cell is within one of the exact
+        // one (unless all_exact)
         bool exact_cell_sum = false;
         if constexpr (SIGNED) {
           if (nxt > u) {
-            int cj[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              long long j;
-              if constexpr (NODES) j = signbit(d32[k]) ? C.walk4_dn[k] - wt[k] : wt[k] - C.walk4_up[k];
-              else j = signbit(d32[k]) ? C.walk_dn[k] - wt[k] : wt[k] - C.walk_up[k];
-              cj[k] = (int)min(max(j, 0ll), (long long)C.ax[k].n - 2);
-            }
-            long long fi = ((long long)cj[2] * C.ax[1].n + cj[1]) * C.ax[0].n + cj[0];
+            const int cx = min(max(cj[0], 0), C.ax[0].n - 2), cy = min(max(cj[1], 0), C.ax[1].n - 2),
+                      cz = min(max(cj[2], 0), C.ax[2].n - 2);
+            long long fi = ((long long)cz * C.ax[1].n + cy) * C.ax[0].n + cx;
 #ifdef BIRP_DEBUG_BOUNDS
             if (!bound_ok(fi, C.neg_n, 3)) fi = 0;
 #endif
-            if (__ldg(C.negflag + fi)) {
-              const double s64 = samples_sum64(R.cube, sm.A[lx], sm.B[ly], R.pos[0], R.pos[1], R.pos[2], R.dt,
-                                               first_c + (int)u, first_c + (int)nxt, cj[0], cj[1], cj[2]);
-              acc.add((float)s64);
+            if (all_exact || __ldg(C.negflag + fi)) {
+              float2 s2 = make_float2(0.f, 0.f);
+              run = signed_cell(&R, sm.A[lx], sm.B[ly], first_c + (int)u, first_c + (int)nxt, cx, cy, cz, run, first_c,
+                                &s2);
+              acc.add(s2.x);
+              acc.add(s2.y);
+              if (run.phase == RUN_ENDED) break;
               u = nxt;
               ncell += 1.f;
               exact_cell_sum = true;
+            } else {
+              run.phase = RUN_GOOD;
+              run.n += (int)(nxt - u);
             }
           }
         }
@@ -1246,6 +1313,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
             } else {
               q += dstr[k];
             }
+            if constexpr (SIGNED) cj[k] += signbit(d32[k]) ? -1 : 1;
           }
         }
       }
@@ -1439,7 +1507,22 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
             if (!bound_ok(q - vb, COMPACT ? C.grid_n : 4 * C.rec_f4, 9)) q = vb;
           }
 #endif
-          acc.add(__ldg(q) * (float)(nxt - u));
+          const float v = __ldg(q);
+          if constexpr (SIGNED) {
+            const bool neg = v < 0.f;
+            if (u == 0) run.first_neg = neg;
+            if (neg && run.phase == RUN_GOOD) {
+              run.phase = RUN_ENDED;
+              break;
+            }
+            if (!neg) {
+              run.phase = RUN_GOOD;
+              run.n += nxt - u;
+              acc.add(v * (float)(nxt - u));
+            }
+          } else {
+            acc.add(v * (float)(nxt - u));
+          }
           u = nxt;
         } else if (++guard > cap) {
           break;
@@ -1548,6 +1631,12 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     else march(*R.cmem);
   }
 
+  if constexpr (KIND == SPACE_CUBE && SIGNED) {
+    const int count = max(0, min((b - a) - seg * (((b - a) + S - 1) >> SEGL2), ((b - a) + S - 1) >> SEGL2));
+    const bool mine = lane_in_run(run, count, R.mode, S, seg, lane);
+    if (!mine) acc = Kahan();
+    nsamp = mine ? run.n : 0;
+  }
   if (stats) {
     unsigned int cnt = __reduce_add_sync(0xffffffffu, (unsigned int)nsamp);
     if (lane == 0 && cnt) atomicAdd(&stats->samples, (unsigned long long)cnt);
@@ -1588,11 +1677,23 @@ __global__ void __launch_bounds__(kThreads) render_plain_kernel(const __grid_con
 // each: nearest 4.82 -> 4.58 ms, compact 4.62 -> 4.48 ms; CMEM at its batch
 // class's count was slower with the plain tile shape, 31.1 -> 33.8 ms, and
 // the records and pairs marches no faster).
-template <int INTERP, int AXES, int MINB>
+template <int INTERP, int AXES, int MINB, bool SIGNED = false>
 __global__ void __launch_bounds__(kThreads, MINB) render_plain_cube_kernel(const __grid_constant__ RequestDev req,
                                                                            KernelStats* stats) {
   __shared__ TileSmem sm;
-  render_tile<SPACE_CUBE, INTERP, AXES>(req, blockIdx.x, blockIdx.y, sm, stats);
+  render_tile<SPACE_CUBE, INTERP, AXES, SIGNED>(req, blockIdx.x, blockIdx.y, sm, stats);
+}
+
+// A nearest-mode tile: any layout, cubes with and without negative values.
+__device__ __forceinline__ void render_tile_nearest(const RequestDev& R, int tx, int ty, TileSmem& sm,
+                                                    KernelStats* st) {
+  if (R.has_neg) {
+    if (R.layout != CUBE_RECORDS) render_tile<SPACE_CUBE, NEAREST, AXES_DDA_COMPACT, true>(R, tx, ty, sm, st);
+    else render_tile<SPACE_CUBE, NEAREST, AXES_DDA, true>(R, tx, ty, sm, st);
+  } else {
+    if (R.layout != CUBE_RECORDS) render_tile<SPACE_CUBE, NEAREST, AXES_DDA_COMPACT>(R, tx, ty, sm, st);
+    else render_tile<SPACE_CUBE, NEAREST, AXES_DDA>(R, tx, ty, sm, st);
+  }
 }
 
 // Dispatch over the request's variant.
@@ -1607,10 +1708,8 @@ __device__ void render_tile_any(const RequestDev& R, int tx, int ty, TileSmem& s
     if (R.layout == CUBE_COMPACT) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT>(R, tx, ty, sm, st);
     else if (R.layout == CUBE_PAIRS) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS>(R, tx, ty, sm, st);
     else render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA>(R, tx, ty, sm, st);
-  } else if (R.layout != CUBE_RECORDS) {
-    render_tile<SPACE_CUBE, NEAREST, AXES_DDA_COMPACT>(R, tx, ty, sm, st);
   } else {
-    render_tile<SPACE_CUBE, NEAREST, AXES_DDA>(R, tx, ty, sm, st);
+    render_tile_nearest(R, tx, ty, sm, st);
   }
 }
 
@@ -1661,8 +1760,7 @@ __global__ void __launch_bounds__(kThreads, CLS == BATCH_ANY          ? 1
     } else if constexpr (CLS == BATCH_CMEM) {
       render_tile<SPACE_CMEM, TRILINEAR, AXES_NONE>(R, tx, ty, sm, B.stats, &model);
     } else if constexpr (CLS == BATCH_CUBE_NEAREST) {
-      if (R.layout != CUBE_RECORDS) render_tile<SPACE_CUBE, NEAREST, AXES_DDA_COMPACT>(R, tx, ty, sm, B.stats);
-      else render_tile<SPACE_CUBE, NEAREST, AXES_DDA>(R, tx, ty, sm, B.stats);
+      render_tile_nearest(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_SIGNED) {
       if (R.layout == CUBE_COMPACT) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT, true>(R, tx, ty, sm, B.stats);
       else if (R.layout == CUBE_PAIRS) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, true>(R, tx, ty, sm, B.stats);
@@ -1997,6 +2095,10 @@ cudaError_t launch_render_plain(const RequestDev& h, KernelStats* stats, cudaStr
   else if (h.interp && h.layout == CUBE_PAIRS)
     render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS><<<grid, kThreads, 0, s>>>(h, cp, stats);
   else if (h.interp) render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA><<<grid, kThreads, 0, s>>>(h, cp, stats);
+  else if (h.has_neg && h.layout != CUBE_RECORDS)
+    render_plain_cube_kernel<NEAREST, AXES_DDA_COMPACT, BIRP_NEAREST_MINB, true><<<grid, kThreads, 0, s>>>(h, stats);
+  else if (h.has_neg)
+    render_plain_cube_kernel<NEAREST, AXES_DDA, BIRP_NEAREST_MINB, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.layout != CUBE_RECORDS)
     render_plain_cube_kernel<NEAREST, AXES_DDA_COMPACT, BIRP_NEAREST_MINB><<<grid, kThreads, 0, s>>>(h, stats);
   else render_plain_cube_kernel<NEAREST, AXES_DDA, BIRP_NEAREST_MINB><<<grid, kThreads, 0, s>>>(h, stats);
