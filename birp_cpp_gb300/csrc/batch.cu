@@ -130,23 +130,6 @@ birp_status batch_create(int max_requests, int64_t max_pixels, birp_batch** out)
   if (e != cudaSuccess) return bail(fail(BIRP_ERR_CUDA, "capture: %s", cudaGetErrorString(e)));
   if ((e = cudaGraphInstantiate(&b->exec, b->graph, 0)) != cudaSuccess)
     return bail(fail(BIRP_ERR_CUDA, "graph instantiate: %s", cudaGetErrorString(e)));
-  // the CMEM kernel's node, whose model parameter each launch may set
-  size_t n_nodes = 0;
-  if ((e = cudaGraphGetNodes(b->graph, nullptr, &n_nodes)) != cudaSuccess)
-    return bail(fail(BIRP_ERR_CUDA, "graph nodes: %s", cudaGetErrorString(e)));
-  std::vector<cudaGraphNode_t> nodes(n_nodes);
-  if ((e = cudaGraphGetNodes(b->graph, nodes.data(), &n_nodes)) != cudaSuccess)
-    return bail(fail(BIRP_ERR_CUDA, "graph nodes: %s", cudaGetErrorString(e)));
-  for (cudaGraphNode_t nd : nodes) {
-    cudaGraphNodeType t;
-    cudaKernelNodeParams kp{};
-    if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel &&
-        cudaGraphKernelNodeGetParams(nd, &kp) == cudaSuccess && kp.func == render_batch_function(BATCH_CMEM)) {
-      b->cmem_node = nd;
-      b->cmem_launch = kp;
-    }
-  }
-  if (!b->cmem_node) return bail(fail(BIRP_ERR_CUDA, "batch graph without its CMEM kernel node"));
   *out = b;
   return ok();
 }
@@ -193,29 +176,6 @@ birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* 
     }
     hdr[4 * cls] = k;
     hdr[4 * cls + 1] = first[k];
-  }
-  // one CMEM model for every CMEM request: the CMEM kernel gets it as a
-  // parameter (its constants become operands instead of loads)
-  const birp_cmem* model = nullptr;
-  bool one_model = true;
-  for (int i = 0; i < n; ++i)
-    if (reqs[i].cmem) {
-      if (!model) model = reqs[i].cmem;
-      else if (reqs[i].cmem != model) one_model = false;
-    }
-  CmemParam cp{};
-  if (model && one_model) {
-    cp.m = model->h_desc;
-    cp.dev = model->d_desc;
-  }
-  if (std::memcmp(&cp, &b->cmem_model, sizeof cp) != 0) {
-    cudaKernelNodeParams kp = b->cmem_launch;
-    void* args[2] = {&b->bd[BATCH_CMEM], &cp};
-    kp.kernelParams = args;
-    kp.extra = nullptr;
-    cudaError_t e = cudaGraphExecKernelNodeSetParams(b->exec, b->cmem_node, &kp);
-    if (e != cudaSuccess) return fail(BIRP_ERR_CUDA, "CMEM model parameter: %s", cudaGetErrorString(e));
-    b->cmem_model = cp;
   }
   b->n = n;
   b->used = used;

@@ -34,11 +34,6 @@ struct birp_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   birp::BatchDev bd[birp::BATCH_CLASSES] = {};  // the kernels' work tables
-  // the CMEM class kernel's node: its CMEM model parameter is set before a
-  // launch whose CMEM requests share one model
-  cudaGraphNode_t cmem_node = nullptr;
-  cudaKernelNodeParams cmem_launch{};
-  birp::CmemParam cmem_model{};  // the parameter the node holds now
   cudaEvent_t e_start = nullptr, e_kernel = nullptr, e_end = nullptr;
 };
 

@@ -106,17 +106,15 @@ struct CmemDev {
   float bc0, bc1, bc3, cos_tn, sin_tn, cos_ts, sin_ts;
   double d_p0, d_p1, d_p2, d_p3, d_dn, d_ds, d_tn, d_ts, d_r0, d_charlie, d_a5, d_a21;
   double d_bs, d_ay, d_az, d_A1, d_A2, d_B, d_alpha, d_beta, d_bc0, d_bc1, d_bc3;
+  double d_cos_tn, d_sin_tn, d_cos_ts, d_sin_ts;
   float eps_rel;  // FP32 boundary-decision margin (relative to r)
+  // Bounds of the two shell surfaces by direction (device, cmem_table_kernel):
+  // kCmemCt x kCmemCp entries over cos theta (fastest) and cos phi
+  // (cmem_table_index), each {r_mp min, r_mp max, r_bs min, r_bs max} over its
+  // directions and a little around them; infinite where they are not known.
+  const float4* table;
 };
-
-// A CMEM model passed by value as a kernel parameter: the kernels that take
-// one read its constants as parameter operands (no loads) for the requests
-// whose model is `dev`; other requests (dev == nullptr: all) read theirs
-// through RequestDev::cmem.
-struct CmemParam {
-  CmemDev m;
-  const CmemDev* dev;
-};
+constexpr int kCmemCt = 256, kCmemCp = 64;
 
 enum SpaceKind : int { SPACE_CUBE = 0, SPACE_CMEM = 1 };
 // Device layouts of a cube (the values of BIRP_CUBE_*).
@@ -178,10 +176,7 @@ struct BatchDev {
 };
 
 // Host-side launch helpers (render.cu).
-// cmem_host: the host copy of req's CMEM model (CMEM requests), passed to the
-// kernel as a parameter
-cudaError_t launch_render_plain(const RequestDev& req, KernelStats* stats, cudaStream_t stream,
-                                const CmemDev* cmem_host = nullptr);
+cudaError_t launch_render_plain(const RequestDev& req, KernelStats* stats, cudaStream_t stream);
 // Persistent-kernel classes: trilinear cube requests in the records layout
 // (fewer registers, more resident warps than the general kernel), the same in
 // the compact and in the pairs layout, CMEM requests, nearest-mode cube
@@ -199,13 +194,7 @@ enum BatchClass : int {
   BATCH_CUBE_TRI_PAIRS = 6,
   BATCH_CLASSES = 7
 };
-// model: the CMEM model the CMEM class kernel takes as a parameter (nullptr:
-// none, every request reads its model through its pointer)
-cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t stream, int cls = BATCH_ANY,
-                                const CmemParam* model = nullptr);
-// The persistent kernel of class cls (its launch's function, for finding its
-// node in a captured graph).
-const void* render_batch_function(int cls);
+cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t stream, int cls = BATCH_ANY);
 int persistent_grid(int cls);
 cudaError_t launch_cube_fill(const float* src_xfast, int nx, int ny, int nz, float* dst, cudaStream_t stream);
 // node values (x fastest; device memory or pinned host memory the device
@@ -223,6 +212,8 @@ cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const
                               cudaStream_t stream);
 cudaError_t launch_cube_sample(const CubeDev* cube, int trilinear, const float* xyz, int n, float* out,
                                cudaStream_t stream);
+// fills cmem->table from the model's coefficients
+cudaError_t launch_cmem_table(const CmemDev* cmem, float4* table, cudaStream_t stream);
 cudaError_t launch_cmem_sample(const CmemDev* cmem, const float* xyz, int n, float* out, cudaStream_t stream);
 cudaError_t launch_cmem_radii_check(const CmemDev* cmem, int n, unsigned long long seed, float* max_err,
                                     cudaStream_t stream);

@@ -495,16 +495,22 @@ birp_status birp_cmem_create(const birp_cmem_params* p, birp_cmem** out) {
   *out = nullptr;
   birp_cmem* m = new birp_cmem();
   cmem_coefficients(*p, m->h_desc);
-  cudaError_t e = cudaMalloc(&m->d_desc, sizeof(CmemDev));
+  // one allocation: the descriptor, then its table of surface bounds
+  constexpr size_t table_off = (sizeof(CmemDev) + 255) / 256 * 256;
+  cudaError_t e = cudaMalloc(&m->d_desc, table_off + sizeof(float4) * kCmemCt * kCmemCp);
   if (e != cudaSuccess) {
     delete m;
     return fail(BIRP_ERR_NOMEM, "cudaMalloc: %s", cudaGetErrorString(e));
   }
-  e = cudaMemcpy(m->d_desc, &m->h_desc, sizeof(CmemDev), cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
+  float4* table = reinterpret_cast<float4*>(reinterpret_cast<char*>(m->d_desc) + table_off);
+  m->h_desc.table = table;
+  if ((e = cudaMemcpyAsync(m->d_desc, &m->h_desc, sizeof(CmemDev), cudaMemcpyHostToDevice, g_ctx.stream)) !=
+          cudaSuccess ||
+      (e = launch_cmem_table(m->d_desc, table, g_ctx.stream)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(g_ctx.stream)) != cudaSuccess) {
     cudaFree(m->d_desc);
     delete m;
-    return fail(BIRP_ERR_CUDA, "cudaMemcpy: %s", cudaGetErrorString(e));
+    return fail(BIRP_ERR_CUDA, "CMEM upload: %s", cudaGetErrorString(e));
   }
   *out = m;
   return ok();
@@ -610,7 +616,7 @@ birp_status birp_render_device(const birp_cube* cube, const birp_cmem* cmem, con
   if (!out_device) return fail(BIRP_ERR_INVALID, "out_device is NULL");
   RequestDev r;
   if (birp_status s = build_request(cube, cmem, *cam, out_device, r)) return s;
-  CK(launch_render_plain(r, g_ctx.stats, pick_stream(stream), cmem ? &cmem->h_desc : nullptr));
+  CK(launch_render_plain(r, g_ctx.stats, pick_stream(stream)));
   return ok();
 }
 
@@ -627,11 +633,11 @@ birp_status birp_render(const birp_cube* cube, const birp_cmem* cmem, const birp
     // the kernel writes every pixel of the caller's image itself
     if (birp_status s = build_request(cube, cmem, *cam, out_host, r)) return s;
     prefault_outputs(&out_host, &npx, 1);
-    CK(launch_render_plain(r, g_ctx.stats, st, cmem ? &cmem->h_desc : nullptr));
+    CK(launch_render_plain(r, g_ctx.stats, st));
   } else {
     if (birp_status s = ensure_scratch(npx)) return s;
     if (birp_status s = build_request(cube, cmem, *cam, g_ctx.scratch, r)) return s;
-    CK(launch_render_plain(r, g_ctx.stats, st, cmem ? &cmem->h_desc : nullptr));
+    CK(launch_render_plain(r, g_ctx.stats, st));
     CK(cudaMemcpyAsync(out_host, g_ctx.scratch, npx * sizeof(float), cudaMemcpyDeviceToHost, st));
   }
   CK(cudaStreamSynchronize(st));
@@ -654,7 +660,7 @@ birp_status birp_time_render_device(const birp_cube* cube, const birp_cmem* cmem
   for (int i = 0; i < repeats; ++i) {
     if (flush_l2) CK(cudaMemsetAsync(g_ctx.flush, i & 0xff, flush_bytes, st));
     CK(cudaEventRecord(e0, st));
-    CK(launch_render_plain(r, g_ctx.stats, st, cmem ? &cmem->h_desc : nullptr));
+    CK(launch_render_plain(r, g_ctx.stats, st));
     CK(cudaEventRecord(e1, st));
     CK(cudaEventSynchronize(e1));
     float ms = 0.f;

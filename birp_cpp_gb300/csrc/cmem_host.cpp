@@ -82,6 +82,10 @@ void cmem_coefficients(const birp_cmem_params& g, CmemDev& m) {
   m.d_ds = ds;
   m.d_tn = tn;
   m.d_ts = ts;
+  m.d_cos_tn = std::cos(tn);
+  m.d_sin_tn = std::sin(tn);
+  m.d_cos_ts = std::cos(ts);
+  m.d_sin_ts = std::sin(ts);
   m.d_r0 = r0;
   m.d_charlie = charlie;
   m.d_a5 = a[5];

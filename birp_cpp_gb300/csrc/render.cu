@@ -431,6 +431,19 @@ __device__ __forceinline__ void cmem_radii32(const CmemDev& m, const CmemDir& d,
   r_bs = cmem_bow_shock(m, d);
 }
 
+// Entry of the table of surface bounds for a direction (cos theta, cos phi,
+// each in [-1, 1] up to rounding). Along an axis of n places entry i, 0 <= i <
+// n - 1, holds c (n/2 - 0.51) + n/2 - 1 in [i - 1/2, i + 1/2]: the sum rounds to
+// kMagic + i, whose low byte is i. The low bytes are put together and masked:
+// the entry is in the table whatever the arguments.
+static_assert(kCmemCt == 256 && (kCmemCp & (kCmemCp - 1)) == 0 && kCmemCp <= 256, "an entry's number is two bytes");
+constexpr float kCtScale = 0.5f * kCmemCt - 0.51f, kCpScale = 0.5f * kCmemCp - 0.51f;
+__device__ __forceinline__ unsigned cmem_table_index(float ct, float cp) {
+  const unsigned i = __float_as_uint(fmaf(ct, kCtScale, kMagic + (0.5f * kCmemCt - 1.f)));
+  const unsigned j = __float_as_uint(fmaf(cp, kCpScale, kMagic + (0.5f * kCmemCp - 1.f)));
+  return __byte_perm(i, j, 0x1140) & (kCmemCt * kCmemCp - 1);
+}
+
 __device__ __forceinline__ CmemEval cmem_value32(const CmemDev& m, float x, float y, float z, float perr) {
   CmemDir d = cmem_dir32_partial(x, y, z);
   const float r = d.r;
@@ -521,43 +534,133 @@ __device__ __forceinline__ CmemEval cmem_value32(const CmemDev& m, float x, floa
   return out;
 }
 
-// The same in FP64 with the FP64 oracle's formulas (oracle cmem64_sample).
-// (not inlined: the fallback is rare, and inlining it would raise the
-// register count of every loop that may call it)
-__device__ __noinline__ double cmem_value64(const CmemDev& m, double x, double y, double z) {
-  const double pi = 3.14159265358979323846;
-  double r = sqrt(x * x + y * y + z * z);
-  double theta = (x != 0) ? acos(x / r) : 0.0;
-  double phi = (y != 0) ? acos(y / sqrt(y * y + z * z)) : 0.0;
-  double phi_n = acos(cos(theta) * cos(m.d_tn) + sin(theta) * sin(m.d_tn) * cos(phi - pi / 2));
-  double phi_s = acos(cos(theta) * cos(m.d_ts) + sin(theta) * sin(m.d_ts) * cos(phi - 3 * pi / 2));
-  double sp = sin(phi);
-  double f = pow(cos(theta / 2) + m.d_a5 * sin(2 * theta) * (1 - exp(-theta)),
-                 m.d_p1 * (m.d_bc0 + m.d_bc1 * cos(phi) + m.d_bc3 * (sp * sp)));
-  double q = m.d_p2 * m.d_charlie * exp(m.d_p3 * m.d_dn * pow(phi_n, m.d_a21)) +
-             m.d_p2 * m.d_charlie * exp(m.d_p3 * m.d_ds * pow(phi_s, m.d_a21));
-  double r_mp = m.d_p0 * m.d_r0 * f + q;
-  double bb = 2 / (1 + cos(theta));
-  double ry = m.d_bs * pow(bb, m.d_ay), rz = m.d_bs * pow(bb, m.d_az);
-  double a1 = rz * cos(phi), a2 = ry * sin(phi);
-  double r_bs = (ry * rz) / sqrt(a1 * a1 + a2 * a2);
-  const double half = (double)(0.05f / 2);
-  double hh = theta / 2, s = sin(theta);
-  double sheath = m.d_A1 * exp(-m.d_B * (hh * hh * hh * hh)) * pow(r / 10, -m.d_alpha - m.d_beta * (s * s));
-  double d10 = r / 10;
-  double outer = m.d_A2 * (1 / (d10 * d10 * d10));
-  if (r < r_mp - half) return 0.0;
-  if (r >= r_mp - half && r <= r_mp + half) {
-    double t = (r - (r_mp - half)) / (r_mp + half);
-    return t * sheath;  // lerp(0, b1, t)
-  }
-  if (r > r_mp + half && r < r_bs - half) return sheath;
-  if (r >= r_bs - half && r <= r_bs + half) {
-    double t = (r - (r_bs - half)) / (r_bs + half);
-    return sheath + t * (outer - sheath);
-  }
-  return outer;
+// Most samples lie well inside a shell: they are decided by the model's table
+// of surface bounds (CmemDev::table) instead of by the radii themselves. With
+// the same half thickness + tol on the sample's side as cmem_value32, a sample
+// below every r_mp of its table entry is in shell 0, one above them all and
+// below every r_bs in shell 2, one above every r_bs too in shell 4: the
+// decision of the full computation, whose value follows from r and theta
+// alone. Returns false (the full computation decides) next to a surface, next
+// to the Earth-Sun line (ryz2 <= off_axis), and for x = 0 or y = 0, whose
+// angles the reference sets to 0.
+// Sheath value: exp(-B (theta/2)^4) multiplies it by 1 - 6 B at most, and B
+// is the field in tesla (~1e-8), so theta to 7e-5 is enough (the table's
+// r_bs bounds say so: unknown where B > 1e-5): acos by Abramowitz and Stegun
+// 4.4.45, |error| <= 6.8e-5.
+// Bound by instruction issue (~62 a sample, from ~205 through the radii; 2 %
+// of the samples still take those). 12 orbit views (2.67e9 samples) 14.1 ->
+// 5.2 ms, a 144x144 view of 200 samples 149 -> 67 us, with the FP64 samples
+// evaluated side by side (cmem_value64). Entries: 128, 256 or 512 over cos
+// theta and 64, 128 or 256 over cos phi within 2 % of each other.
+struct CmemFast {
+  const float4* table;
+  float eps_rel, A1, nB, n_alpha, n_beta, A2k;  // nB = -log2(e) B, A2k = 1000 A2
+};
+__device__ __forceinline__ CmemFast cmem_fast(const CmemDev& m) {
+  return {m.table, m.eps_rel, m.A1, -kLog2e * m.B, -m.alpha, -m.beta, 1000.f * m.A2};
 }
+// half thickness + tol at radius r is fma(eps_rel, r, edge)
+__device__ __forceinline__ float cmem_edge(const CmemFast& m, float perr) { return 0.025f + fmaf(5.f, m.eps_rel, perr); }
+// (x, y, z finite and below 1e15)
+__device__ __forceinline__ bool cmem_by_table(const CmemFast& m, float x, float y, float z, float edge, float off_axis,
+                                              float& v) {
+  const float ryz2 = fmaxf(fmaf(y, y, z * z), 1e-30f), r2 = fmaf(x, x, ryz2);
+  const float ir = rsqrt_fast(r2), r = r2 * ir, ct = x * ir, cp = y * rsqrt_fast(ryz2);
+  const float4 e = __ldg(m.table + cmem_table_index(ct, cp));  // r_mp, r_mp, r_bs, r_bs: min, max
+  const float h = fmaf(m.eps_rel, r, edge), up = r + h, lo = r - h;
+  const bool known = ryz2 > off_axis && x * y != 0.f;
+  const bool past = lo > e.y, in0 = up < e.x, in2 = known && past && up < e.z, in4 = past && lo > e.w;
+  v = in0 ? 0.f : m.A2k * (ir * ir * ir);
+  if (in2) {
+    const float c = fabsf(ct);
+    float p = fmaf(c, -0.0187293f, 0.0742610f);
+    p = fmaf(p, c, -0.2121144f);
+    p = fmaf(p, c, 1.5707288f);
+    const float t = sqrt_fast(fmaxf(1.f - c, 0.f)) * p, hh = 0.5f * (ct < 0.f ? 3.14159274f - t : t);
+    const float h4 = (hh * hh) * (hh * hh), st2 = ryz2 * ir * ir;
+    // log2(r / 10) as half the log2 of (r / 10)^2
+    v = m.A1 * ex2_fast(fmaf(m.nB, h4, fmaf(m.n_beta, st2, m.n_alpha) * (0.5f * __log2f(r2 * 0.01f))));
+  }
+  return in2 || (known && (in0 || in4));
+}
+
+// The same in FP64 for the lanes of a warp that need it, whole warps only: the
+// FP64 oracle's formulas (oracle cmem64_sample), with the direction's cosines
+// and sines taken from the position instead of through acos (equal to ~1e-16;
+// the reference's theta = 0 at x = 0 and phi = 0 at y = 0 kept). An FP64
+// instruction costs a warp the same for 1 lane as for 32, so 8 lanes share a
+// sample: its acos, exp, pow and exp calls each run once, every lane of the
+// group on another argument (4 calls in a row instead of 28; 4 samples at a
+// time). Returns each needing lane its own value.
+__device__ __noinline__ double cmem_value64(const CmemDev& m, bool need, double px, double py, double pz) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, role = lane & 7, base = lane & 24;
+  const double half = (double)(0.05f / 2);
+  double mine = 0.0;
+  for (unsigned todo = __ballot_sync(kAll, need); todo != 0;) {
+    // this group's sample: the todo's (lane / 8)-th lane (its first, unused, when there are fewer)
+    unsigned t = todo;
+    for (int j = 0; j < base; j += 8) t &= t - 1;
+    const int owner = t ? __ffs(t) - 1 : -1, src = t ? owner : __ffs(todo) - 1;
+    const double x = __shfl_sync(kAll, px, src), y = __shfl_sync(kAll, py, src), z = __shfl_sync(kAll, pz, src);
+    auto of = [&](double v, int r) { return __shfl_sync(kAll, v, base + r); };  // lane r of the group
+    const double ryz2 = y * y + z * z, r = sqrt(x * x + ryz2), ryz = sqrt(ryz2);
+    const double ct = x != 0 ? x / r : 1.0, st = x != 0 ? ryz / r : 0.0;
+    const double cp = y != 0 ? y / ryz : 1.0, sp = y != 0 ? fabs(z) / ryz : 0.0;
+    // 2 / (1 + cos theta) without its cancellation towards the tail
+    const double bb = x == 0 ? 1.0 : x > 0 ? 2 * r / (r + x) : 2 * r * (r - x) / ryz2;
+    // angles: theta, and phi_n, phi_s to the cusp axes (cos(phi - pi/2) = sin
+    // phi, cos(phi - 3 pi/2) = -sin phi)
+    const double angle = acos(role == 0   ? ct
+                              : role == 1 ? ct * m.d_cos_tn + st * m.d_sin_tn * sp
+                                          : ct * m.d_cos_ts - st * m.d_sin_ts * sp);
+    const double theta = x != 0 ? of(angle, 0) : 0.0, hh = theta / 2;
+    const double ex1 = exp(role == 0 ? -m.d_B * (hh * hh * hh * hh) : -theta);
+    const double fb = sqrt(1 / bb) + m.d_a5 * (2 * st * ct) * (1 - of(ex1, 1));
+    const double pw = pow(role == 0   ? r / 10
+                          : role <= 2 ? angle
+                          : role == 3 ? fb
+                                      : bb,
+                          role == 0   ? -m.d_alpha - m.d_beta * (st * st)
+                          : role <= 2 ? m.d_a21
+                          : role == 3 ? m.d_p1 * (m.d_bc0 + m.d_bc1 * cp + m.d_bc3 * (sp * sp))
+                          : role == 4 ? m.d_ay
+                                      : m.d_az);
+    const double ex2 = exp((role == 1 ? m.d_p3 * m.d_dn : m.d_p3 * m.d_ds) * pw);
+    const double q = m.d_p2 * m.d_charlie * of(ex2, 1) + m.d_p2 * m.d_charlie * of(ex2, 2);
+    const double r_mp = m.d_p0 * m.d_r0 * of(pw, 3) + q;
+    const double ry = m.d_bs * of(pw, 4), rz = m.d_bs * of(pw, 5);
+    const double a1 = rz * cp, a2 = ry * sp;
+    const double r_bs = (ry * rz) / sqrt(a1 * a1 + a2 * a2);
+    const double sheath = m.d_A1 * of(ex1, 0) * of(pw, 0);
+    const double d10 = r / 10, outer = m.d_A2 * (1 / (d10 * d10 * d10));
+    double v;
+    if (r < r_mp - half) v = 0.0;
+    else if (r >= r_mp - half && r <= r_mp + half) v = (r - (r_mp - half)) / (r_mp + half) * sheath;  // lerp(0, sheath, t)
+    else if (r > r_mp + half && r < r_bs - half) v = sheath;
+    else if (r >= r_bs - half && r <= r_bs + half) v = sheath + (r - (r_bs - half)) / (r_bs + half) * (outer - sheath);
+    else v = outer;
+    for (int j = 0; j < 32; j += 8) {
+      const int o = __shfl_sync(kAll, owner, j);
+      const double w = __shfl_sync(kAll, v, j);
+      if (lane == o) mine = w;
+      todo &= todo - 1;
+    }
+  }
+  return mine;
+}
+
+// The samples of a tile that FP32 leaves open, kept until the tile's march is
+// done and then evaluated in FP64 side by side: a warp's FP64 instruction
+// takes the pipe as long for one lane as for 32, and a call inside the march
+// costs it registers. Each thread has kOpen places; a march that fills them
+// pauses for the tile to evaluate and goes on.
+constexpr int kOpen = 4;
+struct CmemOpen {
+  int n;                                  // filled places of the tile
+  unsigned short list[kThreads * kOpen];  // the places, packed
+  int at[kThreads * kOpen];               // sample index; then the value's bits
+};
 
 // ---------------------------------------------------------------- cube lookup
 
@@ -833,15 +936,13 @@ enum Axes { AXES_NONE = 0, AXES_DDA = 2, AXES_DDA_COMPACT = 3, AXES_DDA_PAIRS = 
 // One pixel tile of one request. The lanes-per-ray split S = 2^seg_log2 is a
 // runtime value of the request (it only sets the tile shape, the lane -> ray
 // map, the sample stride and the merge); the march itself is S-independent.
-// P: a CMEM model passed as a kernel parameter (nullptr: none); CMEM
-// requests whose model it is read its constants from the parameter space.
 // SIGNED: the trilinear march of a cube holding negative values, which sums
 // the cells next to a negative node in float-float (signed_cell) and finds the
 // run's ends there; the nearest march of such a cube finds them by the cells'
 // own values.
 template <int KIND, int INTERP, int AXES, bool SIGNED = false>
 __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty, TileSmem& sm,
-                                            KernelStats* stats, const CmemParam* P = nullptr) {
+                                            KernelStats* stats) {
   const int SEGL2 = R.seg_log2;
   const int S = 1 << SEGL2;
   const int WBXL2 = R.wbx_l2, WGXL2 = R.wgx_l2;
@@ -898,7 +999,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
   const int N = R.N;
   int a = 0, b = N;
   // per-lane telemetry, summed over the warp at the end (one atomic per warp)
-  unsigned int n_exact = 0, n_cells = 0, n_exact_nearest = 0;
+  unsigned int n_exact = 0, n_cells = 0, n_exact_nearest = 0, n_exact_cmem = 0;
   if constexpr (KIND == SPACE_CUBE) {
     const CubeDev& C = *R.cube;
     AxisEst est[3];
@@ -1210,8 +1311,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
                                 &s2);
               acc.add(s2.x);
               acc.add(s2.y);
-              if (run.phase == RUN_ENDED) break;
-              u = nxt;
+              u = run.phase == RUN_ENDED ? ub : nxt;  // (no break: the lanes would not meet again)
               ncell += 1.f;
               exact_cell_sum = true;
             } else {
@@ -1581,54 +1681,95 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     // of the FP64 position at any distance along the ray (an FP32 direction
     // would put a sample t * 1e-7 Re off, a large relative error near the
     // Earth, where the model's values are largest).
-    float st[3], bs[3], st_lo[3], bs_lo[3];
-    {
-      FF wf[3];
+    __shared__ CmemOpen open;
+    const CmemDev& model = *R.cmem;
+    const float end = (float)(first + (iters << SEGL2));
+    for (;;) {
+      int mine = 0;  // this thread's filled places
+      if (tid == 0) open.n = 0;
+      // (from the tile's terms in shared memory in each pass: kept over the FP64
+      // evaluation these registers would be reloaded from the stack by every
+      // sample)
+      float st[3], bs[3], st_lo[3], bs_lo[3];
+      {
+        FF wf[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float h = (float)w64[k];
-        wf[k] = {h, (float)(w64[k] - (double)h)};
-      }
-      const FF rs = ff_rsqrt(ff_add(ff_add(ff_mul(wf[0], wf[0]), ff_mul(wf[1], wf[1])), ff_mul(wf[2], wf[2])));
-      const FF dtf = {R.dt_hi, R.dt_lo};
+        for (int k = 0; k < 3; ++k) {
+          const double w = __dadd_rn(sm.A[lx][k], sm.B[ly][k]);
+          const float h = (float)w;
+          wf[k] = {h, (float)(w - (double)h)};
+        }
+        const FF rs = ff_rsqrt(ff_add(ff_add(ff_mul(wf[0], wf[0]), ff_mul(wf[1], wf[1])), ff_mul(wf[2], wf[2])));
+        const FF dtf = {R.dt_hi, R.dt_lo};
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const FF s2 = ff_mul(ff_mul(wf[k], rs), dtf);
-        const FF b2 = ff_add({R.pos_hi[k], R.pos_lo[k]}, {0.5f * s2.hi, 0.5f * s2.lo});
-        st[k] = s2.hi;
-        st_lo[k] = s2.lo;
-        bs[k] = b2.hi;
-        bs_lo[k] = b2.lo;
+        for (int k = 0; k < 3; ++k) {
+          const FF s2 = ff_mul(ff_mul(wf[k], rs), dtf);
+          const FF b2 = ff_add({R.pos_hi[k], R.pos_lo[k]}, {0.5f * s2.hi, 0.5f * s2.lo});
+          st[k] = s2.hi;
+          st_lo[k] = s2.lo;
+          bs[k] = b2.hi;
+          bs_lo[k] = b2.lo;
+        }
       }
-    }
-    // bound on |x32 - x64| of a sample: two FP32 roundings of a coordinate
-    // (the reach of the ray bounds every coordinate) and the float pairs'
-    // own error
-    const float reach = fabsf(R.pos32[0]) + fabsf(R.pos32[1]) + fabsf(R.pos32[2]) + 1.8f * (float)N * R.dt32;
-    const float perr = fmaf(1.2e-7f, reach, 1e-9f);
-    auto march = [&](const CmemDev& M) {
+      // bound on |x32 - x64| of a sample: two FP32 roundings of a coordinate
+      // (the reach of the ray bounds every coordinate) and the float pairs'
+      // own error
+      const float reach = fabsf(R.pos32[0]) + fabsf(R.pos32[1]) + fabsf(R.pos32[2]) + 1.8f * (float)N * R.dt32;
+      const float perr = fmaf(1.2e-7f, reach, 1e-9f);
+      // directions this far off the Earth-Sun line have cos theta and cos phi
+      // well inside the table's overlap for any position error within perr
+      // (and none where a ray's reach would leave the table's number range)
+      const float off_axis = reach < 1e15f ? fmaxf(1.6e7f * perr * perr, 1e-30f) : INFINITY;
+      const CmemFast M = cmem_fast(model);
+      const float edge = cmem_edge(M, perr);
+      // (the loop's one exit is its condition: with a break in the branch the
+      // warp's lanes do not come together again after it)
+      float stop = end;
 #pragma unroll 1
-      for (int it = 0; it < iters; ++it) {
-        float x = fmaf(fi, st[0], bs[0]) + fmaf(fi, st_lo[0], bs_lo[0]);
-        float y = fmaf(fi, st[1], bs[1]) + fmaf(fi, st_lo[1], bs_lo[1]);
-        float z = fmaf(fi, st[2], bs[2]) + fmaf(fi, st_lo[2], bs_lo[2]);
-        CmemEval e = cmem_value32(M, x, y, z, perr);
-        float v = e.v;
-        if (e.unsure) {
-          need_d64();
-          int i = first + (it << SEGL2);
-          v = (float)cmem_value64(M, pos64(R.pos[0], d64[0], R.dt, i), pos64(R.pos[1], d64[1], R.dt, i),
-                                  pos64(R.pos[2], d64[2], R.dt, i));
-          if (stats) atomicAdd(&stats->exact_cmem, 1ull);
+      while (fi < stop) {
+        const float x = fmaf(fi, st[0], bs[0]) + fmaf(fi, st_lo[0], bs_lo[0]);
+        const float y = fmaf(fi, st[1], bs[1]) + fmaf(fi, st_lo[1], bs_lo[1]);
+        const float z = fmaf(fi, st[2], bs[2]) + fmaf(fi, st_lo[2], bs_lo[2]);
+        float v;
+        if (!cmem_by_table(M, x, y, z, edge, off_axis, v)) {
+          const CmemEval e = cmem_value32(model, x, y, z, perr);
+          v = e.v;
+          if (e.unsure) {
+            v = 0.f;
+            open.at[tid * kOpen + mine] = (int)fi;
+            if (++mine == kOpen) stop = fi;
+          }
         }
         acc.add(v);
         fi += fS;
       }
-    };
-    // the model's constants as parameter operands where the kernel was given
-    // this request's model (one uniform branch per tile), else loaded
-    if (P != nullptr && R.cmem == P->dev) march(P->m);
-    else march(*R.cmem);
+      __syncthreads();
+      if (mine > 0) {
+        const int k = atomicAdd(&open.n, mine);
+        for (int j = 0; j < mine; ++j) open.list[k + j] = (unsigned short)(tid * kOpen + j);
+      }
+      __syncthreads();
+      // place k goes to thread k's position in the order 4 to each warp
+      for (int k0 = 0, n = open.n; k0 < n; k0 += kThreads) {
+        const int k = k0 + (lane >> 2) * 16 + warp * 4 + (lane & 3);
+        const bool need = k < n;
+        if (!__any_sync(0xffffffffu, need)) continue;
+        const int p = open.list[need ? k : k0], t = p / kOpen, i = open.at[p];
+        const int tw = t >> 5, tr = (t & 31) >> SEGL2;
+        const double* ta = sm.A[((tw & (WGX - 1)) << WBXL2) + (tr & (WBX - 1))];
+        const double* tb = sm.B[(tw >> WGXL2) * WBY + (tr >> WBXL2)];
+        double w[3], d[3];
+        for (int r = 0; r < 3; ++r) w[r] = __dadd_rn(ta[r], tb[r]);
+        dir64(w, d);
+        const double v = cmem_value64(model, need, pos64(R.pos[0], d[0], R.dt, i), pos64(R.pos[1], d[1], R.dt, i),
+                                      pos64(R.pos[2], d[2], R.dt, i));
+        if (need) open.at[p] = __float_as_int((float)v);
+      }
+      const bool more = __syncthreads_or(fi < end);
+      for (int j = 0; j < mine; ++j) acc.add(__int_as_float(open.at[tid * kOpen + j]));
+      n_exact_cmem += mine;
+      if (!more) break;
+    }
   }
 
   if constexpr (KIND == SPACE_CUBE && SIGNED) {
@@ -1646,6 +1787,8 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     if (lane == 0 && cc) atomicAdd(&stats->cells, (unsigned long long)cc);
     const unsigned int cn = __reduce_add_sync(0xffffffffu, n_exact_nearest);
     if (lane == 0 && cn) atomicAdd(&stats->exact_nearest, (unsigned long long)cn);
+    const unsigned int cm = __reduce_add_sync(0xffffffffu, n_exact_cmem);
+    if (lane == 0 && cm) atomicAdd(&stats->exact_cmem, (unsigned long long)cm);
   }
   // merge the S partial sums of a ray
   float hi = acc.s, lo = -acc.c;
@@ -1662,21 +1805,17 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
 }
 
 // One request, one CTA per tile; the request travels as a kernel parameter.
-// CMEM requests also get their model as a parameter.
 template <int KIND, int INTERP, int AXES, bool SIGNED = false>
 __global__ void __launch_bounds__(kThreads) render_plain_kernel(const __grid_constant__ RequestDev req,
-                                                                const __grid_constant__ CmemParam model,
                                                                 KernelStats* stats) {
   __shared__ TileSmem sm;
-  render_tile<KIND, INTERP, AXES, SIGNED>(req, blockIdx.x, blockIdx.y, sm, stats,
-                                          KIND == SPACE_CMEM ? &model : nullptr);
+  render_tile<KIND, INTERP, AXES, SIGNED>(req, blockIdx.x, blockIdx.y, sm, stats);
 }
 
 // The nearest and compact-layout trilinear marches alone, compiled for the
 // resident CTAs per SM of their batch classes (16 orbit renders, one call
-// each: nearest 4.82 -> 4.58 ms, compact 4.62 -> 4.48 ms; CMEM at its batch
-// class's count was slower with the plain tile shape, 31.1 -> 33.8 ms, and
-// the records and pairs marches no faster).
+// each: nearest 4.82 -> 4.58 ms, compact 4.62 -> 4.48 ms; the records and
+// pairs marches no faster).
 template <int INTERP, int AXES, int MINB, bool SIGNED = false>
 __global__ void __launch_bounds__(kThreads, MINB) render_plain_cube_kernel(const __grid_constant__ RequestDev req,
                                                                            KernelStats* stats) {
@@ -1720,8 +1859,6 @@ __device__ void render_tile_any(const RequestDev& R, int tx, int ty, TileSmem& s
 // registers, more resident warps); BATCH_CUBE_SIGNED the trilinear march of
 // cubes holding negative values (any layout); BATCH_ANY renders every
 // request kind.
-// `model`: the CMEM class kernel reads this CMEM model's constants as
-// parameter operands for the requests that use it (model.dev).
 template <int CLS>
 __global__ void __launch_bounds__(kThreads, CLS == BATCH_ANY          ? 1
                                            : CLS == BATCH_CMEM         ? BIRP_CMEM_MINB
@@ -1730,7 +1867,7 @@ __global__ void __launch_bounds__(kThreads, CLS == BATCH_ANY          ? 1
                                            : CLS == BATCH_CUBE_TRI_PAIRS ? BIRP_PAIRS_MINB
                                            : CLS == BATCH_CUBE_SIGNED  ? BIRP_SIGNED_MINB
                                                                        : BIRP_WALK_MINB)
-    render_batch_kernel(BatchDev B, const __grid_constant__ CmemParam model) {
+    render_batch_kernel(BatchDev B) {
   __shared__ TileSmem sm;
   __shared__ int s_item;
   const int n_reqs = __ldg(B.hdr), total_items = __ldg(B.hdr + 1);
@@ -1758,7 +1895,7 @@ __global__ void __launch_bounds__(kThreads, CLS == BATCH_ANY          ? 1
     } else if constexpr (CLS == BATCH_CUBE_TRI_PAIRS) {
       render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CMEM) {
-      render_tile<SPACE_CMEM, TRILINEAR, AXES_NONE>(R, tx, ty, sm, B.stats, &model);
+      render_tile<SPACE_CMEM, TRILINEAR, AXES_NONE>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_NEAREST) {
       render_tile_nearest(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_SIGNED) {
@@ -1944,11 +2081,100 @@ __global__ void cube_sample_kernel(const CubeDev* __restrict__ cube, int triline
 
 __global__ void cmem_sample_kernel(const CmemDev* __restrict__ cmem, const float* __restrict__ xyz, int n,
                                    float* __restrict__ out) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    float x = xyz[3 * t], y = xyz[3 * t + 1], z = xyz[3 * t + 2];
-    CmemEval e = cmem_value32(*cmem, x, y, z, 1e-6f);
-    out[t] = e.unsure ? (float)cmem_value64(*cmem, x, y, z) : e.v;
+  const CmemFast fast = cmem_fast(*cmem);
+  const float edge = cmem_edge(fast, 1e-6f);
+  for (int w = blockIdx.x * blockDim.x + (threadIdx.x & ~31); w < n; w += gridDim.x * blockDim.x) {  // whole warps
+    const int t = min(w + (int)(threadIdx.x & 31), n - 1);
+    const float x = xyz[3 * t], y = xyz[3 * t + 1], z = xyz[3 * t + 2];
+    const bool far = !(fabsf(x) + fabsf(y) + fabsf(z) < 1e15f);  // or not a number
+    float v = 0.f;
+    bool open = false;
+    if (far || !cmem_by_table(fast, x, y, z, edge, 1.6e-5f, v)) {
+      const CmemEval e = cmem_value32(*cmem, x, y, z, 1e-6f);
+      v = e.v;
+      open = e.unsure;
+    }
+    if (__any_sync(0xffffffffu, open)) {
+      const double d = cmem_value64(*cmem, open, x, y, z);
+      if (open) v = (float)d;
+    }
+    out[t] = v;
   }
+}
+
+// The table of surface bounds (CmemDev::table): r_mp and r_bs over each
+// entry's directions by interval arithmetic (every factor of cmem_mp_base,
+// cmem_cusps and cmem_bow_shock is monotone or bounded by its end values),
+// over an overlap of 1e-3 in cos theta and cos phi around the entry and
+// widened by more than the FP32 rounding of the bounds themselves. One entry
+// per thread, once per model (about 10 us).
+struct Span {
+  float lo, hi;
+};
+__device__ __forceinline__ Span span_mul(Span a, Span b) {
+  const float p = a.lo * b.lo, q = a.lo * b.hi, r = a.hi * b.lo, s = a.hi * b.hi;
+  return {fminf(fminf(p, q), fminf(r, s)), fmaxf(fmaxf(p, q), fmaxf(r, s))};
+}
+__device__ __forceinline__ Span span_add(Span a, Span b) { return {a.lo + b.lo, a.hi + b.hi}; }
+__device__ __forceinline__ Span span_of(float a) { return {a, a}; }
+__device__ __forceinline__ Span span_sqr(Span a) {
+  const float p = a.lo * a.lo, q = a.hi * a.hi;
+  return {a.lo <= 0.f && a.hi >= 0.f ? 0.f : fminf(p, q), fmaxf(p, q)};
+}
+
+__global__ void cmem_table_kernel(const CmemDev* __restrict__ cmem, float4* __restrict__ table) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= kCmemCt * kCmemCp) return;
+  const CmemDev& m = *cmem;
+  const float pad = 1e-3f, pi = 3.14159274f;
+  auto cosines = [&](int i, int n, float scale) -> Span {
+    return {fmaxf((i + 0.5f - 0.5f * n) / scale - pad, -1.f), fminf((i + 1.5f - 0.5f * n) / scale + pad, 1.f)};
+  };
+  const Span ct = cosines(t % kCmemCt, kCmemCt, kCtScale), cp = cosines(t / kCmemCt, kCmemCp, kCpScale);
+  const Span th = {acosf(ct.hi), acosf(ct.lo)}, ph = {acosf(cp.hi), acosf(cp.lo)};
+  const Span ct2 = span_sqr(ct), cp2 = span_sqr(cp);
+  const Span st = {sqrtf(1.f - ct2.hi), sqrtf(1.f - ct2.lo)}, sp2 = {1.f - cp2.hi, 1.f - cp2.lo};
+  // r_mp = p0 r0 f + q
+  const Span ch = {sqrtf(0.5f * (1.f + ct.lo)), sqrtf(0.5f * (1.f + ct.hi))};
+  const Span s2e = span_mul(span_mul(st, ct), {1.f - expf(-th.lo), 1.f - expf(-th.hi)});
+  const Span base = span_add(ch, span_mul(s2e, span_of(2.f * m.a5)));
+  const Span ex = span_mul(span_of(m.p1),
+                           span_add(span_of(m.bc0), span_add(span_mul(cp, span_of(m.bc1)), span_mul(sp2, span_of(m.bc3)))));
+  Span mp = {-INFINITY, INFINITY};
+  if (base.lo > 1e-3f) {
+    const Span lf = span_mul(ex, {log2f(base.lo), log2f(base.hi)});
+    mp = span_mul(span_of(m.p0r0), {exp2f(lf.lo), exp2f(lf.hi)});
+    // the angle to a cusp axis: within the entry's reach of its value at the
+    // middle (reach: along the meridian, then along the parallel)
+    const float thc = 0.5f * (th.lo + th.hi), phc = 0.5f * (ph.lo + ph.hi);
+    const float reach = 0.5f * (th.hi - th.lo) + st.hi * 0.5f * (ph.hi - ph.lo) + 1e-3f;
+    for (int s = 0; s < 2; ++s) {
+      const float ca = s ? m.cos_ts : m.cos_tn, sa = s ? -m.sin_ts : m.sin_tn, k = s ? m.p3ds : m.p3dn;
+      const float c = cosf(thc) * ca + sinf(thc) * sinf(phc) * sa;
+      const float a = acosf(fminf(fmaxf(c, -1.f), 1.f));
+      const Span an = {fmaxf(a - reach, 0.f), fminf(a + reach, pi)};
+      const float p = powf(an.lo, m.a21), q = powf(an.hi, m.a21);
+      const Span g = span_mul(span_of(k), {fminf(p, q), fmaxf(p, q)});
+      mp = span_add(mp, span_mul(span_of(m.p2c), {expf(g.lo), expf(g.hi)}));
+    }
+  }
+  // 1 / r_bs^2 = (cos phi / ry)^2 + (sin phi / rz)^2
+  Span bs = {-INFINITY, INFINITY};
+  if (ct.lo > -0.999f && m.bs > 0.f) {
+    const Span lb = {1.f - log2f(1.f + ct.hi), 1.f - log2f(1.f + ct.lo)};
+    const Span ly = span_mul(span_of(-2.f * m.ay), lb), lz = span_mul(span_of(-2.f * m.az), lb);
+    const Span inv = span_add(span_mul(cp2, {exp2f(ly.lo), exp2f(ly.hi)}), span_mul(sp2, {exp2f(lz.lo), exp2f(lz.hi)}));
+    bs = {m.bs * rsqrtf(inv.hi), m.bs * rsqrtf(inv.lo)};
+  }
+  auto widen = [](Span a) -> Span {
+    if (!(a.lo <= a.hi)) return {-INFINITY, INFINITY};  // NaN
+    return {a.lo - 2e-4f * (fabsf(a.lo) + 5.f), a.hi + 2e-4f * (fabsf(a.hi) + 5.f)};
+  };
+  mp = widen(mp);
+  bs = widen(bs);
+  // a sheath value needs theta to full precision where B is not small
+  if (!(m.B <= 1e-5f)) bs.lo = -INFINITY;
+  table[t] = make_float4(mp.lo, mp.hi, bs.lo, bs.hi);
 }
 
 // Validates the FP32 CMEM boundary-radius error bound: max over n pseudo-
@@ -2075,26 +2301,21 @@ bool tile_shape_ok(int segl2, int wbx_l2, int wgx_l2) {
 }
 int default_wbx_l2(int segl2) { return segl2 == 0 ? 3 : segl2 <= 2 ? 2 : segl2 <= 4 ? 1 : 0; }
 
-cudaError_t launch_render_plain(const RequestDev& h, KernelStats* stats, cudaStream_t s, const CmemDev* cmem_host) {
+cudaError_t launch_render_plain(const RequestDev& h, KernelStats* stats, cudaStream_t s) {
   const int tw = tile_w(h.seg_log2, h.wbx_l2, h.wgx_l2), th = tile_h(h.seg_log2, h.wbx_l2, h.wgx_l2);
   dim3 grid((h.nx + tw - 1) / tw, (h.ny + th - 1) / th);
-  CmemParam cp{};
-  if (h.kind == SPACE_CMEM && cmem_host) {
-    cp.m = *cmem_host;
-    cp.dev = h.cmem;
-  }
-  if (h.kind == SPACE_CMEM) render_plain_kernel<SPACE_CMEM, TRILINEAR, AXES_NONE><<<grid, kThreads, 0, s>>>(h, cp, stats);
+  if (h.kind == SPACE_CMEM) render_plain_kernel<SPACE_CMEM, TRILINEAR, AXES_NONE><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.has_neg && h.layout == CUBE_COMPACT)
-    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT, true><<<grid, kThreads, 0, s>>>(h, cp, stats);
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.has_neg && h.layout == CUBE_PAIRS)
-    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, true><<<grid, kThreads, 0, s>>>(h, cp, stats);
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.has_neg)
-    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA, true><<<grid, kThreads, 0, s>>>(h, cp, stats);
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.layout == CUBE_COMPACT)
     render_plain_cube_kernel<TRILINEAR, AXES_DDA_COMPACT, BIRP_COMPACT_MINB><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.layout == CUBE_PAIRS)
-    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS><<<grid, kThreads, 0, s>>>(h, cp, stats);
-  else if (h.interp) render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA><<<grid, kThreads, 0, s>>>(h, cp, stats);
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS><<<grid, kThreads, 0, s>>>(h, stats);
+  else if (h.interp) render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.has_neg && h.layout != CUBE_RECORDS)
     render_plain_cube_kernel<NEAREST, AXES_DDA_COMPACT, BIRP_NEAREST_MINB, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.has_neg)
@@ -2127,27 +2348,15 @@ int persistent_grid(int cls) {
   return sms * per_sm;
 }
 
-cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t s, int cls, const CmemParam* model) {
-  CmemParam cp{};
-  if (model) cp = *model;
-  if (cls == BATCH_CUBE_TRI) render_batch_kernel<BATCH_CUBE_TRI><<<grid, kThreads, 0, s>>>(b, cp);
-  else if (cls == BATCH_CUBE_TRI_COMPACT) render_batch_kernel<BATCH_CUBE_TRI_COMPACT><<<grid, kThreads, 0, s>>>(b, cp);
-  else if (cls == BATCH_CUBE_TRI_PAIRS) render_batch_kernel<BATCH_CUBE_TRI_PAIRS><<<grid, kThreads, 0, s>>>(b, cp);
-  else if (cls == BATCH_CMEM) render_batch_kernel<BATCH_CMEM><<<grid, kThreads, 0, s>>>(b, cp);
-  else if (cls == BATCH_CUBE_NEAREST) render_batch_kernel<BATCH_CUBE_NEAREST><<<grid, kThreads, 0, s>>>(b, cp);
-  else if (cls == BATCH_CUBE_SIGNED) render_batch_kernel<BATCH_CUBE_SIGNED><<<grid, kThreads, 0, s>>>(b, cp);
-  else render_batch_kernel<BATCH_ANY><<<grid, kThreads, 0, s>>>(b, cp);
+cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t s, int cls) {
+  if (cls == BATCH_CUBE_TRI) render_batch_kernel<BATCH_CUBE_TRI><<<grid, kThreads, 0, s>>>(b);
+  else if (cls == BATCH_CUBE_TRI_COMPACT) render_batch_kernel<BATCH_CUBE_TRI_COMPACT><<<grid, kThreads, 0, s>>>(b);
+  else if (cls == BATCH_CUBE_TRI_PAIRS) render_batch_kernel<BATCH_CUBE_TRI_PAIRS><<<grid, kThreads, 0, s>>>(b);
+  else if (cls == BATCH_CMEM) render_batch_kernel<BATCH_CMEM><<<grid, kThreads, 0, s>>>(b);
+  else if (cls == BATCH_CUBE_NEAREST) render_batch_kernel<BATCH_CUBE_NEAREST><<<grid, kThreads, 0, s>>>(b);
+  else if (cls == BATCH_CUBE_SIGNED) render_batch_kernel<BATCH_CUBE_SIGNED><<<grid, kThreads, 0, s>>>(b);
+  else render_batch_kernel<BATCH_ANY><<<grid, kThreads, 0, s>>>(b);
   return cudaGetLastError();
-}
-
-const void* render_batch_function(int cls) {
-  if (cls == BATCH_CUBE_TRI) return (const void*)render_batch_kernel<BATCH_CUBE_TRI>;
-  if (cls == BATCH_CUBE_TRI_COMPACT) return (const void*)render_batch_kernel<BATCH_CUBE_TRI_COMPACT>;
-  if (cls == BATCH_CUBE_TRI_PAIRS) return (const void*)render_batch_kernel<BATCH_CUBE_TRI_PAIRS>;
-  if (cls == BATCH_CMEM) return (const void*)render_batch_kernel<BATCH_CMEM>;
-  if (cls == BATCH_CUBE_NEAREST) return (const void*)render_batch_kernel<BATCH_CUBE_NEAREST>;
-  if (cls == BATCH_CUBE_SIGNED) return (const void*)render_batch_kernel<BATCH_CUBE_SIGNED>;
-  return (const void*)render_batch_kernel<BATCH_ANY>;
 }
 
 bool read_bounds_status(unsigned long long* status, bool reset) {
@@ -2210,6 +2419,12 @@ cudaError_t launch_cube_sample(const CubeDev* cube, int trilinear, const float* 
   if (n <= 0) return cudaSuccess;
   int blocks = std::min((n + 255) / 256, 4096);
   cube_sample_kernel<<<blocks, 256, 0, s>>>(cube, trilinear, xyz, n, out);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_cmem_table(const CmemDev* cmem, float4* table, cudaStream_t s) {
+  const int n = kCmemCt * kCmemCp;
+  cmem_table_kernel<<<(n + 127) / 128, 128, 0, s>>>(cmem, table);
   return cudaGetLastError();
 }
 
