@@ -689,32 +689,6 @@ __device__ int exact_cell(const AxisDev& a, double x, int guess) {
   return k;
 }
 
-// First sample index i in [lo, hi] past the plane c along one axis, by the
-// FP64 oracle's own position pos64(i) = p + d ((i + 1/2) dt): moving up, past
-// means pos64 >= c; moving down, pos64 < c (hi if none in [lo, hi)). The
-// predicate is monotone in i. Not inlined: it runs only when a float-float
-// crossing lies within its error bound of an integer.
-__device__ __noinline__ int exact_first_past(double p, double d, double dt, double c, bool up, int lo, int hi) {
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    const double x = pos64(p, d, dt, mid);
-    if (up ? (x >= c) : (x < c)) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
-// The same, with the ray's FP64 direction rebuilt from the tile's column and
-// row terms (a, b: the oracle's w = a + b, normalised as dir64 does), so the
-// caller's walk keeps no FP64 state live.
-__device__ __noinline__ int exact_first_past_ray(const double* a, const double* b, int axis, double p, double dt,
-                                                 double c, bool up, int lo, int hi) {
-  double w[3], d[3];
-  for (int r = 0; r < 3; ++r) w[r] = __dadd_rn(a[r], b[r]);
-  dir64(w, d);
-  return exact_first_past(p, d[axis], dt, c, up, lo, hi);
-}
-
 // ---------------------------------------------------------------- negative values
 
 // std::lerp in FP64 as libstdc++ defines it (the FP64 oracle interpolates with
@@ -897,6 +871,101 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
     }
   }
   *sum = make_float2(s.hi, s.lo);
+  return run;
+}
+
+// First sample index i in [lo, hi] past the plane c along one axis, by the
+// FP64 oracle's own position pos64(i) = p + d ((i + 1/2) dt): moving up, past
+// means pos64 >= c; moving down, pos64 < c (hi if none in [lo, hi)). The
+// predicate is monotone in i.
+__device__ int exact_first_past(double p, double d, double dt, double c, bool up, int lo, int hi) {
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    const double x = pos64(p, d, dt, mid);
+    if (up ? (x >= c) : (x < c)) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
+
+// A lane's nearest samples [i0, i1) where float-float leaves a plane crossing
+// open (a sample on a plane, to ~1e-13 of the coordinates): the walk with
+// every crossing in float-float and, within its bound, by the oracle's FP64
+// predicate. Negative values as in signed_cell. Not inlined: such runs are
+// rare, and a call inside the walk would cost it registers.
+__device__ __noinline__ LaneRun nearest_run_exact(const RequestDev* Rp, const double* a, const double* b, int i0,
+                                                  int i1, float2* sum) {
+  const RequestDev& R = *Rp;
+  const CubeDev& C = *R.cube;
+  LaneRun run{R.mode == MARCH_PREFIX ? RUN_GOOD : RUN_SKIP, false, 0};
+  double w[3], d[3], s = 0.0;
+  for (int r = 0; r < 3; ++r) w[r] = __dadd_rn(a[r], b[r]);
+  dir64(w, d);
+  FF inv[3], K[3];
+  int c[3], nxt[3];
+  const int never = 0x3fffffff;
+  // first sample in [0, N) past the lane's next plane along axis k
+  auto cross = [&](int k) -> int {
+    if (d[k] == 0.0) return never;
+    const bool up = d[k] > 0.0;
+    const int j = up ? c[k] + 1 : c[k];
+    if (j < 0 || j >= C.ax[k].n) return never;  // beyond the box
+    const float2 P = __ldg(C.nodes_ff[k] + j);
+    const FF u = ff_add(ff_mul({P.x, P.y}, inv[k]), {-K[k].hi, -K[k].lo});
+    if (!(u.hi <= (float)R.N + 1.5f)) return never;
+    if (u.hi < -1.5f) return 0;
+    const float n0 = rintf(u.hi), dist = (u.hi - n0) + u.lo;
+    const float cp = fmaxf(fabsf((float)C.ax[k].c_first), fabsf((float)C.ax[k].c_last)) + fabsf(R.pos32[k]);
+    const float E = fmaf(1e-14f * cp, fabsf(inv[k].hi), fmaf(3e-13f, (float)(R.N + 2), 1e-9f));
+    int i;
+    if (fabsf(dist) > E) {
+      i = max((int)n0 + (dist > 0.f ? 1 : 0), 0);
+    } else {
+      const float uc = u.hi + u.lo;
+      i = exact_first_past(R.pos[k], d[k], R.dt, C.ax[k].c64[j], up, max((int)floorf(uc - E) - 1, 0),
+                           min((int)ceilf(uc + E) + 2, R.N));
+    }
+    return i < R.N ? i : never;
+  };
+  for (int k = 0; k < 3; ++k) {
+    FF wf[3];
+    for (int r = 0; r < 3; ++r) wf[r] = {(float)w[r], (float)(w[r] - (double)(float)w[r])};
+    const FF rs = ff_rsqrt(ff_add(ff_add(ff_mul(wf[0], wf[0]), ff_mul(wf[1], wf[1])), ff_mul(wf[2], wf[2])));
+    inv[k] = d[k] != 0.0 ? ff_recip(ff_mul(ff_mul(wf[k], rs), {R.dt_hi, R.dt_lo})) : FF{0.f, 0.f};
+    K[k] = ff_add(ff_mul({R.pos_hi[k], R.pos_lo[k]}, inv[k]), {0.5f, 0.f});
+    const double x = pos64(R.pos[k], d[k], R.dt, i0);
+    int lo = 0, hi = C.ax[k].n - 1;  // largest node at or below x, by bisection
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (C.ax[k].c64[mid] <= x) lo = mid;
+      else hi = mid;
+    }
+    c[k] = lo;
+    nxt[k] = cross(k);
+  }
+  for (int u = i0; u < i1 && run.phase != RUN_ENDED;) {
+    const int n = min(min(min(nxt[0], nxt[1]), nxt[2]), i1);
+    if (n > u) {
+      const double v = node_value(C, c[0], c[1], c[2]);
+      const bool neg = R.has_neg && v < 0.0;
+      if (neg && u == i0) run.first_neg = true;
+      if (!neg) {
+        run.phase = RUN_GOOD;
+        run.n += n - u;
+        s += v * (double)(n - u);
+      } else if (run.phase == RUN_GOOD) {
+        run.phase = RUN_ENDED;
+      }
+      u = n;
+    }
+    for (int k = 0; k < 3; ++k)
+      if (nxt[k] <= u) {  // its plane is passed: the next one
+        c[k] += d[k] > 0.0 ? 1 : -1;
+        nxt[k] = cross(k);
+      }
+  }
+  const float h = (float)s;
+  *sum = make_float2(h, isfinite(h) ? (float)(s - (double)h) : 0.f);
   return run;
 }
 
@@ -1438,7 +1507,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     const int first_c = a + min(seg * seglen, total);
     const int count = max(0, min(total - seg * seglen, seglen));
     nsamp = count;
-    unsigned int n_fp64 = 0;
+    bool open = false;  // a plane crossing that float-float leaves open
     if (count > 0) {
       // Per axis: 1 / (d dt) and K = p / (d dt) + 1/2 as float pairs, so the
       // crossing index of plane P is u = P / (d dt) - K; the error bound E of
@@ -1507,53 +1576,13 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         if (fabsf(dist) > E) {
           i = max((int)n0 + (dist > 0.f ? 1 : 0), 0);
         } else {
-          // within the bound: the oracle's predicate decides
-          ++n_fp64;
-#ifdef BIRP_DEBUG_BOUNDS
-          long long ci = nd - C.nodes_ff[k];
-          if (!bound_ok(ci, C.ax[k].n, 8)) ci = 0;
-          const double c = C.ax[k].c64[ci];
-#else
-          const double c = C.ax[k].c64[nd - C.nodes_ff[k]];
-#endif
-          const float uc = u.hi + u.lo;
-          i = exact_first_past_ray(sm.A[lx], sm.B[ly], k, R.pos[k], R.dt, c, inv[k].hi > 0.f,
-                                   max((int)floorf(uc - E) - 1, 0), min((int)ceilf(uc + E) + 2, N));
-        }
-        return i < N ? i : kNever;
-      };
-      // a crossing whose FP32 estimate was within its bound of an integer,
-      // for the axis k of the walk step (operands chosen by the caller):
-      // float-float, then the oracle's FP64 predicate within that bound
-      auto cross_ff = [&](int k, const float2* nd, FF invk, FF Kk, float cpk) -> int {
-#ifdef BIRP_DEBUG_BOUNDS
-        if (!bound_ok(nd - (C.nodes_ff[0] - 1), C.nodes_n, 8)) nd = C.nodes_ff[0];
-#endif
-        const float2 P = __ldg(nd);
-        const FF u = ff_add(ff_mul({P.x, P.y}, invk), {-Kk.hi, -Kk.lo});
-        const float n0 = rintf(u.hi);
-        const float dist = (u.hi - n0) + u.lo;
-        const float E = fmaf(1e-14f * cpk, fabsf(invk.hi), fmaf(3e-13f, (float)(N + 2), 1e-9f));
-        int i;
-        if (fabsf(dist) > E) {
-          i = max((int)n0 + (dist > 0.f ? 1 : 0), 0);
-        } else {
-          ++n_fp64;
-#ifdef BIRP_DEBUG_BOUNDS
-          long long ci = nd - C.nodes_ff[k];
-          if (!bound_ok(ci, C.ax[k].n, 8)) ci = 0;
-          const double c = C.ax[k].c64[ci];
-#else
-          const double c = C.ax[k].c64[nd - C.nodes_ff[k]];
-#endif
-          const float uc = u.hi + u.lo;
-          i = exact_first_past_ray(sm.A[lx], sm.B[ly], k, R.pos[k], R.dt, c, invk.hi > 0.f,
-                                   max((int)floorf(uc - E) - 1, 0), min((int)ceilf(uc + E) + 2, N));
+          open = true;  // within the bound: the run is walked by nearest_run_exact
+          i = 0;
         }
         return i < N ? i : kNever;
       };
       // the lane's first cell, exactly; then the next plane on each axis
-      int nxtc[3], dstr[3];
+      int ds[3], dn[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const AxisDev& A = C.ax[k];
@@ -1579,99 +1608,139 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
           np[k] = nodes + (up ? kk + 1 : kk);  // the next plane: node kk + 1 up, kk down
         }
         kc[k] = kk;
-        nxtc[k] = cross(k, np[k]) - first_c;
-        const int stride =
-            COMPACT ? (int)record_stride(C.gx, C.gxy, k) << C.gshift : 8 * (int)record_stride(C.cx, C.cxy, k);
-        dstr[k] = up ? stride : -stride;  // in floats
+        const int stride = (int)(COMPACT ? record_stride(C.gx, C.gxy, k) : record_stride(C.cx, C.cxy, k));
+        ds[k] = up ? stride : -stride;  // in cells
+        dn[k] = up ? 1 : -1;
       }
-      // node value pointer: the padded grid (compact, pairs) or the first
-      // float of the cell's record (8 floats); cells stay within [-1, n-1],
-      // whose data exist, because a walk stops at the sentinel planes
-      const float* q = COMPACT ? C.grid + (record_index(C.gx, C.gxy, kc[0], kc[1], kc[2]) << C.gshift)
-                               : reinterpret_cast<const float*>(C.rec) + 8 * record_index(C.cx, C.cxy, kc[0], kc[1], kc[2]);
-      // the next planes as indices into the node table of all three axes
-      // (one allocation: axis k's nodes start at nodes_ff[k])
+      // The walk. Per axis ex is the FP32 crossing index of the next plane, one
+      // FMA a step; a crossing is looked at closely only when it is the next
+      // one and within E of an integer: then float-float (the pairs wait in
+      // shared memory), and within that bound the oracle's predicate, decide
+      // it, and ex becomes (first sample past the plane) - 1/2, certain from
+      // there on. An axis is stepped when its crossing lies before the current
+      // sample by more than E. An axis along which the ray hardly moves (E
+      // above 0.015; 0.005 to 0.03 within 4 %, 0.1 5 % and 0.002 29 % slower)
+      // gets no estimate, and so does not widen E for the others: its ex is
+      // far below any sample, so its plane is always decided closely, and
+      // first of all.
+      // Bound by issue and the close looks' chains (a warp has one in 1 of 8
+      // iterations). 24 orbit renders of the 256^3 cube, pairs layout: 3.97 ms
+      // with one certified crossing per iteration picked by selects, 3.2 ms
+      // so; records 4.12 -> 3.4 ms.
+      __shared__ float pairs[12][kThreads];
+      float ex[3], fi32[3], fK[3], E = 0.f;
+      int ni[3];  // the next planes as indices into the node table of all three axes
       const float2* nbase = C.nodes_ff[0];
-      int ni[3];
 #pragma unroll
-      for (int k = 0; k < 3; ++k) ni[k] = (int)(np[k] - nbase);
-      int u = 0;
-      const int cap = count + C.ax[0].n + C.ax[1].n + C.ax[2].n + 4;
-      int guard = 0;  // iterations that sum nothing (see the trilinear walk)
-      while (u < count) {
-        const int nxt = min(min(min(nxtc[0], nxtc[1]), nxtc[2]), count);
-        if (nxt > u) {
-#ifdef BIRP_DEBUG_BOUNDS
-          {
-            const float* vb = COMPACT ? C.grid : reinterpret_cast<const float*>(C.rec);
-            if (!bound_ok(q - vb, COMPACT ? C.grid_n : 4 * C.rec_f4, 9)) q = vb;
-          }
-#endif
-          const float v = __ldg(q);
-          if constexpr (SIGNED) {
-            const bool neg = v < 0.f;
-            if (u == 0) run.first_neg = neg;
-            if (neg && run.phase == RUN_GOOD) {
-              run.phase = RUN_ENDED;
-              break;
-            }
-            if (!neg) {
-              run.phase = RUN_GOOD;
-              run.n += nxt - u;
-              acc.add(v * (float)(nxt - u));
-            }
-          } else {
-            acc.add(v * (float)(nxt - u));
-          }
-          u = nxt;
-        } else if (++guard > cap) {
-          break;
-        }
-        if (u >= count) break;  // the run is summed: no further steps
-        // step the axis whose plane comes first (its crossing is <= u here; an
-        // axis due at the same sample is stepped next iteration, which sums
-        // nothing): one crossing per iteration, its operands chosen by
-        // selects; an undecided FP32 crossing goes to the full computation
-        const int k = (nxtc[0] <= nxtc[1]) ? (nxtc[0] <= nxtc[2] ? 0 : 2) : (nxtc[1] <= nxtc[2] ? 1 : 2);
-        const int ds = k == 0 ? dstr[0] : (k == 1 ? dstr[1] : dstr[2]);
-        q += ds;
-        const int nk = (k == 0 ? ni[0] : (k == 1 ? ni[1] : ni[2])) + (ds > 0 ? 1 : -1);
-        ni[0] = k == 0 ? nk : ni[0];
-        ni[1] = k == 1 ? nk : ni[1];
-        ni[2] = k == 2 ? nk : ni[2];
+      for (int k = 0; k < 3; ++k) {
+        pairs[4 * k][tid] = inv[k].hi;
+        pairs[4 * k + 1][tid] = inv[k].lo;
+        pairs[4 * k + 2][tid] = K[k].hi;
+        pairs[4 * k + 3][tid] = K[k].lo;
+        const float Ek = fmaf(6.1e-8f, (float)(N + 2), E32[k]);  // and the rounding of u - E below
+        const bool good = Ek <= 0.015f;
+        if (good) E = fmaxf(E, Ek);
+        fi32[k] = good ? inv[k].hi : 0.f;
+        fK[k] = good ? K[k].hi : 3e38f;
+        ni[k] = (int)(np[k] - nbase);
+        ex[k] = w64[k] == 0.0 ? INFINITY : fmaf(__ldg(np[k]).x, fi32[k], -fK[k]);
+      }
+      // first sample past the plane of node index nk along axis k, in
+      // float-float: INFINITY when no sample of the ray is
+      auto close_look = [&](int k, int nk) -> float {
+        const FF invk = {pairs[4 * k][tid], pairs[4 * k + 1][tid]}, Kk = {pairs[4 * k + 2][tid], pairs[4 * k + 3][tid]};
         const float2* nd = nbase + nk;
-        const float invh = k == 0 ? inv[0].hi : (k == 1 ? inv[1].hi : inv[2].hi);
-        const float Kh = k == 0 ? K[0].hi : (k == 1 ? K[1].hi : K[2].hi);
-        const float Ek = k == 0 ? E32[0] : (k == 1 ? E32[1] : E32[2]);
 #ifdef BIRP_DEBUG_BOUNDS
         if (!bound_ok(nd - (C.nodes_ff[0] - 1), C.nodes_n, 8)) nd = C.nodes_ff[0];
 #endif
         const float2 P = __ldg(nd);
-        const float u32 = fmaf(P.x, invh, -Kh);
-        // (the next plane's crossing is never behind the current sample: the
-        // general branch covers u32 < -1.5 too, giving 0)
-        int c;
-        if (!(u32 <= (float)N + 1.5f)) {
-          c = kNever;  // also NaN: a sentinel plane
+        const FF uf = ff_add(ff_mul({P.x, P.y}, invk), {-Kk.hi, -Kk.lo});
+        if (!(uf.hi <= (float)N + 1.5f)) return INFINITY;  // also NaN
+        if (uf.hi < -1.5f) return -0.5f;
+        const float n0 = rintf(uf.hi), dist = (uf.hi - n0) + uf.lo;
+        const float c = fmaxf(fabsf((float)C.ax[k].c_first), fabsf((float)C.ax[k].c_last)) + fabsf(R.pos32[k]);
+        // the bound of `cross` above
+        const float Ef = fmaf(1e-14f * c, fabsf(invk.hi), fmaf(3e-13f, (float)(N + 2), 1e-9f));
+        int i;
+        if (fabsf(dist) > Ef) {
+          i = max((int)n0 + (dist > 0.f ? 1 : 0), 0);
         } else {
-          const float m0 = rintf(u32);
-          const float d32u = u32 - m0;
-          if (fabsf(d32u) > Ek) {
-            const int i = max((int)m0 + (d32u > 0.f ? 1 : 0), 0);
-            c = i < N ? i : kNever;
-          } else {
-            const FF ik = {invh, k == 0 ? inv[0].lo : (k == 1 ? inv[1].lo : inv[2].lo)};
-            const FF kk2 = {Kh, k == 0 ? K[0].lo : (k == 1 ? K[1].lo : K[2].lo)};
-            c = cross_ff(k, nd, ik, kk2, k == 0 ? cp[0] : (k == 1 ? cp[1] : cp[2]));
+          open = true;
+          return INFINITY;
+        }
+        return i < N ? (float)i - 0.5f : INFINITY;
+      };
+      // node value of the cell: the padded grid (compact, pairs) or the first
+      // float of the cell's record; cells stay within [-1, n-1], whose data
+      // exist, because a walk never steps over a sentinel plane (its crossing
+      // is infinite)
+      const char* vbase = reinterpret_cast<const char*>(COMPACT ? C.grid : reinterpret_cast<const float*>(C.rec));
+      const unsigned vbytes = COMPACT ? 4u << C.gshift : 32u;
+      unsigned cell = (unsigned)(COMPACT ? record_index(C.gx, C.gxy, kc[0], kc[1], kc[2])
+                                         : record_index(C.cx, C.cxy, kc[0], kc[1], kc[2]));
+      float u = (float)first_c;
+      const float ub = open ? u : (float)(first_c + count);
+      // (one exit: a break inside a branch would keep the lanes apart; ends
+      // because an iteration without samples steps an axis, and an axis has
+      // at most n steps before its infinite crossing)
+      for (;;) {
+        float exm = fminf(fminf(ex[0], ex[1]), ex[2]);
+        // (at most once per axis: a decided crossing is half an index from any integer)
+        for (int tries = 0; tries < 3 && exm < ub + 1.f && !(fabsf((ceilf(exm) - exm) - 0.5f) < 0.5f - E); ++tries) {
+          const int k = ex[0] == exm ? 0 : ex[1] == exm ? 1 : 2;
+          const float e = close_look(k, k == 0 ? ni[0] : k == 1 ? ni[1] : ni[2]);
+          ex[0] = k == 0 ? e : ex[0];
+          ex[1] = k == 1 ? e : ex[1];
+          ex[2] = k == 2 ? e : ex[2];
+          exm = fminf(fminf(ex[0], ex[1]), ex[2]);
+        }
+        const float nxt = fmaxf(fminf(ceilf(exm), ub), u), m = nxt - u;
+#ifdef BIRP_DEBUG_BOUNDS
+        if (!bound_ok((long long)cell * (vbytes / 4), COMPACT ? C.grid_n : 4 * C.rec_f4, 9)) cell = 0;
+#endif
+        const float v = __ldg(reinterpret_cast<const float*>(vbase + (size_t)cell * vbytes));
+        bool good = m > 0.f;
+        u = nxt;
+        if constexpr (SIGNED) {
+          const bool neg = good && v < 0.f;
+          if (neg && m == nxt - (float)first_c) run.first_neg = true;
+          if (neg && run.phase == RUN_GOOD) {
+            run.phase = RUN_ENDED;
+            u = ub;
+          }
+          good = good && !neg;
+          if (good) {
+            run.phase = RUN_GOOD;
+            run.n += (int)m;
           }
         }
-        c -= first_c;
-        nxtc[0] = k == 0 ? c : nxtc[0];
-        nxtc[1] = k == 1 ? c : nxtc[1];
-        nxtc[2] = k == 2 ? c : nxtc[2];
+        acc.add_product(m, good ? v : 0.f);
+        if (u >= ub) break;
+        // (the next crossing is stepped however u - E is rounded)
+        const float past = fmaxf(u - E, exm);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (ex[k] <= past) {
+            ni[k] += dn[k];
+            cell += (unsigned)ds[k];
+            const float2* nd = nbase + ni[k];
+#ifdef BIRP_DEBUG_BOUNDS
+            if (!bound_ok(nd - (C.nodes_ff[0] - 1), C.nodes_n, 8)) nd = C.nodes_ff[0];
+#endif
+            ex[k] = fmaf(__ldg(&nd->x), fi32[k], -fK[k]);
+          }
+        }
       }
     }
-    n_exact_nearest = n_fp64;
+    if (open) {
+      float2 s2;
+      const LaneRun r = nearest_run_exact(&R, sm.A[lx], sm.B[ly], first_c, first_c + count, &s2);
+      if constexpr (SIGNED) run = r;
+      acc = Kahan();
+      acc.add(s2.x);
+      acc.add(s2.y);
+      n_exact_nearest = count;
+    }
   } else {
     // Sample positions p + d ((i + 1/2) dt) from the ray's exact direction:
     // the step d dt and the first position as float pairs (hi + lo, ~48-bit
