@@ -454,15 +454,38 @@ birp_status birp_cube_get_info(const birp_cube* cube, birp_cube_info* info) {
   return ok();
 }
 
+// Whether a sampling call's arrays can be read and written by the kernel where
+// they lie: host memory the device accesses (as birp_render), apart from each
+// other (a result written over a point still to be read needs the copies).
+static bool direct_points(const float* xyz, const float* out, size_t n) {
+  if (!host_direct_writes() || (xyz < out + n && out < xyz + 3 * n)) return false;
+  for (const void* p : {(const void*)xyz, (const void*)out}) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (a.type == cudaMemoryTypeDevice) return false;  // refused by the copies
+  }
+  return true;
+}
+
 birp_status birp_cube_sample(const birp_cube* cube, int trilinear, const float* xyz, int n, float* out) {
   if (birp_status s = check_init()) return s;
   if (!cube || (n > 0 && (!xyz || !out)) || n < 0) return fail(BIRP_ERR_INVALID, "bad argument");
   if (n == 0) return ok();
+  cudaStream_t st = g_ctx.stream;
+  if (direct_points(xyz, out, (size_t)n)) {
+    const size_t count = (size_t)n;
+    prefault_outputs(&out, &count, 1);
+    CK(launch_cube_sample(cube->d_desc, trilinear, xyz, n, out, st));
+    CK(cudaStreamSynchronize(st));
+    return ok();
+  }
   std::lock_guard<std::mutex> lk(g_ctx.mu);
   if (birp_status s = ensure_xyz_scratch((size_t)n * 4)) return s;
   float* d_xyz = g_ctx.xyz_scratch;
   float* d_out = d_xyz + (size_t)3 * n;
-  cudaStream_t st = g_ctx.stream;
   CK(cudaMemcpyAsync(d_xyz, xyz, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, st));
   CK(launch_cube_sample(cube->d_desc, trilinear, d_xyz, n, d_out, st));
   CK(cudaMemcpyAsync(out, d_out, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
@@ -528,11 +551,18 @@ birp_status birp_cmem_sample(const birp_cmem* m, const float* xyz, int n, float*
   if (birp_status s = check_init()) return s;
   if (!m || (n > 0 && (!xyz || !out)) || n < 0) return fail(BIRP_ERR_INVALID, "bad argument");
   if (n == 0) return ok();
+  cudaStream_t st = g_ctx.stream;
+  if (direct_points(xyz, out, (size_t)n)) {
+    const size_t count = (size_t)n;
+    prefault_outputs(&out, &count, 1);
+    CK(launch_cmem_sample(m->d_desc, xyz, n, out, st));
+    CK(cudaStreamSynchronize(st));
+    return ok();
+  }
   std::lock_guard<std::mutex> lk(g_ctx.mu);
   if (birp_status s = ensure_xyz_scratch((size_t)n * 4)) return s;
   float* d_xyz = g_ctx.xyz_scratch;
   float* d_out = d_xyz + (size_t)3 * n;
-  cudaStream_t st = g_ctx.stream;
   CK(cudaMemcpyAsync(d_xyz, xyz, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, st));
   CK(launch_cmem_sample(m->d_desc, d_xyz, n, d_out, st));
   CK(cudaMemcpyAsync(out, d_out, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
