@@ -197,18 +197,21 @@ enum BatchClass : int {
 cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t stream, int cls = BATCH_ANY);
 int persistent_grid(int cls);
 cudaError_t launch_cube_fill(const float* src_xfast, int nx, int ny, int nz, float* dst, cudaStream_t stream);
-// node values (x fastest; device memory or pinned host memory the device
-// reads) into the interior of the padded grid
-cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, cudaStream_t stream);
+// node values (x fastest; device memory or host memory the device reads) into
+// the interior of the padded grid; *neg (device, nullptr: not wanted) becomes 1
+// if one is below zero
+cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, int* neg, cudaStream_t stream);
 cudaError_t launch_cube_negflags(const float* padded, int nx, int ny, int nz, uint8_t* flags, cudaStream_t stream);
 // bounds-checking build: the first out-of-range access (code << 48 | index),
 // 0 if none, optionally reset; other builds: always 0, returns false
 bool read_bounds_status(unsigned long long* status, bool reset);
-cudaError_t launch_cube_records(const float* padded, int nx, int ny, int nz, const double* cx64, const double* cy64,
-                                const double* cz64, float4* rec, cudaStream_t stream);
+// iwx, iwy, iwz: the inverse widths of cells -1..n-1 (0 for the guard cells) as
+// float pairs (device)
+cudaError_t launch_cube_records(const float* padded, int nx, int ny, int nz, const float2* iwx, const float2* iwy,
+                                const float2* iwz, float4* rec, cudaStream_t stream);
 // the pairs layout's {value, z-slope} per padded node (padded: the guard-filled
-// scalar grid; cz64: the FP64 z coordinates)
-cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const double* cz64, float2* pairs,
+// scalar grid)
+cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const float2* iwz, float2* pairs,
                               cudaStream_t stream);
 cudaError_t launch_cube_sample(const CubeDev* cube, int trilinear, const float* xyz, int n, float* out,
                                cudaStream_t stream);

@@ -459,6 +459,7 @@ birp_status birp_cube_get_info(const birp_cube* cube, birp_cube_info* info) {
 // other (a result written over a point still to be read needs the copies).
 static bool direct_points(const float* xyz, const float* out, size_t n) {
   if (!host_direct_writes() || (xyz < out + n && out < xyz + 3 * n)) return false;
+  if (((uintptr_t)xyz | (uintptr_t)out) % alignof(float) != 0) return false;
   for (const void* p : {(const void*)xyz, (const void*)out}) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {

@@ -139,8 +139,18 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   const size_t px = (size_t)nx + 2, py = (size_t)ny + 2, pz = (size_t)nz + 2;
   const size_t total = px * py * pz;
   const size_t nodes = (size_t)nx * ny * nz;
-  if (c.has_neg < 0) c.has_neg = any_negative(values, nodes) ? 1 : 0;
   if (!st) st = g_ctx.stream;
+  // Where the device accesses the values it reads them itself, and finds out on
+  // the way whether one is below zero: pinned host memory (the server's
+  // copies), and pageable memory on a host whose memory is coherent with the
+  // device. Other memory goes by one strided 3D copy, its signs scanned here.
+  cudaPointerAttributes pa{};
+  const bool known = cudaPointerGetAttributes(&pa, values) == cudaSuccess;
+  cudaGetLastError();  // (an unregistered pointer is not an error to keep)
+  const bool direct = ((uintptr_t)values % alignof(float)) == 0 && known &&
+                      (pa.type == cudaMemoryTypeHost || (pa.type == cudaMemoryTypeUnregistered && host_direct_writes()));
+  const bool find_neg = direct && c.has_neg < 0;
+  if (c.has_neg < 0) c.has_neg = !direct && any_negative(values, nodes) ? 1 : 0;
   c.alloc_stream = stream_alloc ? st : nullptr;
 
   CubeDev& d = c.h_desc;
@@ -198,8 +208,22 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   // the padded scalar grid; records and pairs layouts: turned into records
   // (pairs), then freed (held in d_grid until then, so a failed upload
   // releases it with the rest)
+  // (followed by the inverse widths of cells -1..n-1 per axis, as float pairs,
+  // and the sign the copy finds)
   float* scalar = nullptr;
-  CKU(dev_alloc(&scalar, total * sizeof(float), c.alloc_stream));
+  std::vector<float2> iw;
+  if (!compact) {
+    iw.reserve(coords + 3);
+    for (int k = 0; k < 3; ++k)
+      for (int j = -1; j < c.n[k]; ++j) {
+        const double w = j >= 0 && j + 1 < c.n[k] ? 1.0 / (c.c[k][j + 1] - c.c[k][j]) : 0.0;
+        iw.push_back(make_float2((float)w, (float)(w - (double)(float)w)));
+      }
+  }
+  const size_t iw_off = (total * sizeof(float) + 7) / 8 * 8, neg_off = iw_off + iw.size() * sizeof(float2);
+  CKU(dev_alloc(&scalar, neg_off + (find_neg ? sizeof(int) : 0), c.alloc_stream));
+  float2* const d_iw = reinterpret_cast<float2*>(reinterpret_cast<char*>(scalar) + iw_off);
+  int* const d_neg = find_neg ? reinterpret_cast<int*>(reinterpret_cast<char*>(scalar) + neg_off) : nullptr;
   c.d_grid = scalar;
   if (nodes_layout) {
     CKU(dev_alloc(&c.d_walk4, walk.size() * sizeof(float4), c.alloc_stream));
@@ -223,14 +247,10 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
                     : pairs ? total * sizeof(float2) + walk.size() * sizeof(float4)
                             : records * 2 * sizeof(float4) + walk2.size() * sizeof(float2));
 
-  // interior values from the caller's x-fastest array: pinned host memory
-  // (the server's copies) is read by a kernel straight into the padded grid;
-  // other (pageable) memory goes by one strided 3D copy
-  cudaPointerAttributes pa{};
-  const bool pinned = cudaPointerGetAttributes(&pa, values) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-  cudaGetLastError();  // (an unregistered pointer is not an error to keep)
-  if (pinned) {
-    CKU(launch_cube_pad_copy(values, nx, ny, nz, scalar, st));
+  // interior values from the caller's x-fastest array
+  if (direct) {
+    if (find_neg) CKU(cudaMemsetAsync(d_neg, 0, sizeof(int), st));
+    CKU(launch_cube_pad_copy(values, nx, ny, nz, scalar, d_neg, st));
   } else {
     cudaMemcpy3DParms p;
     std::memset(&p, 0, sizeof p);
@@ -242,7 +262,18 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
     CKU(cudaMemcpy3DAsync(&p, st));
   }
   CKU(launch_cube_fill(nullptr, nx, ny, nz, scalar, st));
+  if (find_neg) {  // before the last use of the grid: a cube with one needs its flags from it
+    int neg = 0;
+    CKU(cudaMemcpyAsync(&neg, d_neg, sizeof neg, cudaMemcpyDeviceToHost, st));
+    CKU(cudaStreamSynchronize(st));
+    c.has_neg = neg;
+    if (neg) {
+      CKU(dev_alloc(&c.d_negflag, nodes, c.alloc_stream));
+      c.device_bytes += nodes;
+    }
+  }
   if (c.has_neg) CKU(launch_cube_negflags(scalar, nx, ny, nz, c.d_negflag, st));
+  if (!iw.empty()) CKU(cudaMemcpyAsync(d_iw, iw.data(), iw.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
   // (the host vectors below stay alive until the synchronize at the end)
   std::vector<double> all;
   all.reserve(coords);
@@ -267,14 +298,14 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   if (nodes_layout) {
     CKU(cudaMemcpyAsync(c.d_walk4, walk.data(), walk.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
     if (pairs) {
-      CKU(launch_cube_pairs(scalar, nx, ny, nz, c.d_c64 + nx + ny, c.d_pairs, st));
+      CKU(launch_cube_pairs(scalar, nx, ny, nz, d_iw + nx + ny + 2, c.d_pairs, st));
       if (c.alloc_stream) {
         c.d_grid = nullptr;
         CKU(cudaFreeAsync(scalar, st));
       }
     }
   } else {
-    CKU(launch_cube_records(scalar, nx, ny, nz, c.d_c64, c.d_c64 + nx, c.d_c64 + nx + ny, c.d_vals, st));
+    CKU(launch_cube_records(scalar, nx, ny, nz, d_iw, d_iw + nx + 1, d_iw + nx + ny + 2, c.d_vals, st));
     if (c.alloc_stream) {
       c.d_grid = nullptr;
       CKU(cudaFreeAsync(scalar, st));

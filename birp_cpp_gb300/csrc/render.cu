@@ -2013,15 +2013,57 @@ __global__ void cube_guard_kernel(float* dst, int nx, int ny, int nz) {
 
 // Copies the x-fastest node values into the interior of the padded grid
 // (node (i, j, k) to padded (i+1, j+1, k+1)), reading the source where it
-// lies: pinned host memory is read by the kernel itself (over NVLink-C2C on a
-// Grace host), one coalesced pass, instead of a strided 3D copy.
-__global__ void cube_pad_copy_kernel(const float* __restrict__ src, int nx, int ny, int nz, float* __restrict__ dst) {
-  const long long n = (long long)nx * ny * nz, px = nx + 2, pxy = (long long)(nx + 2) * (ny + 2);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const long long row = t / nx, x = t - row * nx;
-    const long long y = row % ny, z = row / ny;
-    dst[(z + 1) * pxy + (y + 1) * px + (x + 1)] = __ldcs(src + t);
+// lies: host memory is read by the kernel itself (over NVLink-C2C on a Grace
+// host), 4 values a load from the first 16-byte boundary on. neg, when given,
+// becomes 1 if a value is below zero. Bound by the host link (13.8 M values,
+// 55 MB: 2.0 ms by a strided 3D copy and 2.9 ms of host scan for the sign,
+// 0.27 ms so, 203 GB/s).
+__global__ void cube_pad_copy_kernel(const float* __restrict__ src, unsigned n, int nx, int ny, int nz,
+                                     float* __restrict__ dst, int* __restrict__ neg) {
+  const long long px = nx + 2, pxy = (long long)(nx + 2) * (ny + 2);
+  bool below = false;
+  auto put = [&](unsigned t, float v, unsigned& x, long long& o) {  // value t, then the place of the next
+    dst[o] = v;
+    below |= v < 0.f;
+    ++o;
+    if (++x == (unsigned)nx) {
+      x = 0;
+      const unsigned row = (t + 1) / (unsigned)nx, y = row % (unsigned)ny, z = row / (unsigned)ny;
+      o = (z + 1) * pxy + (y + 1) * px + 1;
+    }
+  };
+  auto place = [&](unsigned t, unsigned& x) -> long long {
+    const unsigned row = t / (unsigned)nx, y = row % (unsigned)ny, z = row / (unsigned)ny;
+    x = t - row * (unsigned)nx;
+    return (z + 1) * pxy + (y + 1) * px + (x + 1);
+  };
+  const unsigned head = min(n, (unsigned)((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4);
+  const unsigned quads = (n - head) / 4, tail = head + 4 * quads;
+  const unsigned id = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+  unsigned x;
+  if (id < head || (id >= 4 && id - 4 < n - tail)) {  // the ends, one value each
+    const unsigned t = id < head ? id : tail + (id - 4);
+    long long o = place(t, x);
+    put(t, src[t], x, o);
   }
+  const float4* s4 = reinterpret_cast<const float4*>(src + head);
+  for (unsigned q0 = id; q0 < quads; q0 += 4 * all) {
+    float4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (q0 + j * all < quads) v[j] = __ldcs(s4 + q0 + j * all);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (q0 + j * all < quads) {
+        const unsigned t = head + 4 * (q0 + j * all);
+        long long o = place(t, x);
+        put(t, v[j].x, x, o);
+        put(t + 1, v[j].y, x, o);
+        put(t + 2, v[j].z, x, o);
+        put(t + 3, v[j].w, x, o);
+      }
+  }
+  if (neg && __any_sync(0xffffffffu, below) && (threadIdx.x & 31) == 0) *neg = 1;
 }
 
 // Cell records from the padded scalar grid ((nx+2)(ny+2)(nz+2), node i at
@@ -2029,61 +2071,115 @@ __global__ void cube_pad_copy_kernel(const float* __restrict__ src, int nx, int 
 // polynomial of the 8 padded nodes (a..a+1, b..b+1, c..c+1) (cell a-1 of the
 // unpadded grid) in local physical coordinates: the fraction coefficients
 // times the inverse cell widths (0 for a guard cell, whose two faces along
-// that axis hold equal values), computed in FP64 and rounded once.
-__device__ __forceinline__ double inv_width(const double* c, int n, long long a) {
-  return (a >= 1 && a <= n - 1) ? 1.0 / (c[a] - c[a - 1]) : 0.0;
+// that axis hold equal values), computed in float-float and rounded once: the
+// first differences are exact pairs, the inverse widths (iw*: one per cell
+// -1..n-1) FP64 values as pairs, so a coefficient is off by one rounding as
+// from FP64, which is 1/58 of the rate. Values or coefficients that leave
+// float-float's range take FP64.
+__device__ __noinline__ void cell_record64(const float* v, const double* i3, float* out) {
+  const double v000 = v[0], v001 = v[1], v010 = v[2], v011 = v[3], v100 = v[4], v101 = v[5], v110 = v[6], v111 = v[7];
+  const double ix = i3[0], iy = i3[1], iz = i3[2];
+  const double c1 = (v001 - v000) * ix, c2 = (v010 - v000) * iy, c3 = (v100 - v000) * iz;
+  const double c4 = ((v011 - v010) - (v001 - v000)) * (ix * iy);
+  const double c5 = ((v101 - v100) - (v001 - v000)) * (ix * iz);
+  const double c6 = ((v110 - v100) - (v010 - v000)) * (iy * iz);
+  const double c7 = (((v111 - v110) - (v101 - v100)) - ((v011 - v010) - (v001 - v000))) * (ix * iy * iz);
+  const double c[8] = {v000, c3, c1, c5, c2, c6, c4, c7};
+  for (int k = 0; k < 8; ++k) out[k] = (float)c[k];
 }
+__device__ __forceinline__ FF ff_diff(float a, float b) {  // a - b, exactly
+  FF r;
+  two_sum(a, -b, r.hi, r.lo);
+  return r;
+}
+__device__ __forceinline__ FF ff_sub(FF a, FF b) { return ff_add(a, {-b.hi, -b.lo}); }
 
-__global__ void cube_records_kernel(const float* __restrict__ v, int nx, int ny, int nz, const double* __restrict__ cx64,
-                                    const double* __restrict__ cy64, const double* __restrict__ cz64,
+// (bound by the store of the records: 13.8 M cells, 440 MB, 1.43 ms with FP64
+// arithmetic, 0.134 ms so, 3.7 TB/s read and written)
+__global__ void cube_records_kernel(const float* __restrict__ v, int nx, int ny, int nz, const float2* __restrict__ iwx,
+                                    const float2* __restrict__ iwy, const float2* __restrict__ iwz,
                                     float4* __restrict__ rec) {
-  const long long cx = nx + 1, cy = ny + 1, cz = nz + 1, px = nx + 2, pxy = (long long)(nx + 2) * (ny + 2);
-  const long long n = cx * cy * cz;
-  for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < n; r += (long long)gridDim.x * blockDim.x) {
-    const long long a = r % cx, b = (r / cx) % cy, c = r / (cx * cy);
+  const unsigned cx = nx + 1, cy = ny + 1;
+  const unsigned n = cx * cy * (unsigned)(nz + 1);
+  const long long px = nx + 2, pxy = (long long)(nx + 2) * (ny + 2);
+  for (unsigned long long r = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; r < n;
+       r += gridDim.x * (unsigned long long)blockDim.x) {
+    const unsigned q = (unsigned)r / cx, a = (unsigned)r - q * cx, c = q / cy, b = q - c * cy;
     const float* p = v + c * pxy + b * px + a;
-    const double v000 = p[0], v001 = p[1], v010 = p[px], v011 = p[px + 1];
-    const double v100 = p[pxy], v101 = p[pxy + 1], v110 = p[pxy + px], v111 = p[pxy + px + 1];
-    const double ix = inv_width(cx64, nx, a), iy = inv_width(cy64, ny, b), iz = inv_width(cz64, nz, c);
-    const double c1 = (v001 - v000) * ix, c2 = (v010 - v000) * iy, c3 = (v100 - v000) * iz;
-    const double c4 = ((v011 - v010) - (v001 - v000)) * (ix * iy);
-    const double c5 = ((v101 - v100) - (v001 - v000)) * (ix * iz);
-    const double c6 = ((v110 - v100) - (v010 - v000)) * (iy * iz);
-    const double c7 = (((v111 - v110) - (v101 - v100)) - ((v011 - v010) - (v001 - v000))) * (ix * iy * iz);
-    rec[2 * r] = make_float4((float)v000, (float)c3, (float)c1, (float)c5);
-    rec[2 * r + 1] = make_float4((float)c2, (float)c6, (float)c4, (float)c7);
+    const float v000 = __ldg(p), v001 = __ldg(p + 1), v010 = __ldg(p + px), v011 = __ldg(p + px + 1);
+    const float v100 = __ldg(p + pxy), v101 = __ldg(p + pxy + 1), v110 = __ldg(p + pxy + px),
+                v111 = __ldg(p + pxy + px + 1);
+    const float2 fx = __ldg(iwx + a), fy = __ldg(iwy + b), fz = __ldg(iwz + c);
+    const FF ix = {fx.x, fx.y}, iy = {fy.x, fy.y}, iz = {fz.x, fz.y};
+    const FF d1 = ff_diff(v001, v000), d2 = ff_diff(v010, v000), d3 = ff_diff(v100, v000);
+    const FF t = ff_diff(v011, v010), w = ff_diff(v101, v100);
+    const FF e4 = ff_sub(t, d1), e5 = ff_sub(w, d1), e6 = ff_sub(ff_diff(v110, v100), d2);
+    const FF e7 = ff_sub(ff_sub(ff_diff(v111, v110), w), e4);
+    const FF ixy = ff_mul(ix, iy);
+    float o[8] = {v000,
+                  ff_mul(d3, iz).hi,
+                  ff_mul(d1, ix).hi,
+                  ff_mul(e5, ff_mul(ix, iz)).hi,
+                  ff_mul(d2, iy).hi,
+                  ff_mul(e6, ff_mul(iy, iz)).hi,
+                  ff_mul(e4, ixy).hi,
+                  ff_mul(e7, ff_mul(ixy, iz)).hi};
+    const float size = fabsf(v000) + fabsf(v001) + fabsf(v010) + fabsf(v011) + fabsf(v100) + fabsf(v101) + fabsf(v110) +
+                       fabsf(v111);
+    float coefs = 0.f;
+#pragma unroll
+    for (int k = 1; k < 8; ++k) coefs += fabsf(o[k]);
+    if (!(size == 0.f || (size > 1e-20f && size < 1e30f && coefs < 1e30f))) {
+      const float f[8] = {v000, v001, v010, v011, v100, v101, v110, v111};
+      const double i3[3] = {(double)fx.x + fx.y, (double)fy.x + fy.y, (double)fz.x + fz.y};
+      cell_record64(f, i3, o);
+    }
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(rec + 2 * r), "f"(o[0]), "f"(o[1]),
+                 "f"(o[2]), "f"(o[3]), "f"(o[4]), "f"(o[5]), "f"(o[6]), "f"(o[7])
+                 : "memory");
   }
 }
 
 // Pairs layout from the padded scalar grid: every padded node (i, j, k) gets
-// {v, s}, s the slope of its z-edge (v(k+1) - v(k)) / (z(k+1) - z(k)) in FP64
-// rounded once (the records layout's c3 of the cell above it, bit for bit),
-// 0 where that cell is a guard cell (its values repeat the edge node).
-__global__ void cube_pairs_kernel(const float* __restrict__ v, int nx, int ny, int nz, const double* __restrict__ cz64,
+// {v, s}, s the slope of its z-edge (v(k+1) - v(k)) / (z(k+1) - z(k)) in
+// float-float rounded once (the records layout's c3 of the cell above it), 0
+// where that cell is a guard cell (its values repeat the edge node). iwz: the
+// inverse widths of cells -1..nz-1, i.e. of padded layers 0..nz.
+__global__ void cube_pairs_kernel(const float* __restrict__ v, int nx, int ny, int nz, const float2* __restrict__ iwz,
                                   float2* __restrict__ pairs) {
-  const long long pxy = (long long)(nx + 2) * (ny + 2);
-  const long long n = pxy * (nz + 2);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const double iz = inv_width(cz64, nz, t / pxy);  // 0 unless the padded layer is 1..nz-1
-    const float v0 = v[t];
-    pairs[t] = make_float2(v0, iz != 0.0 ? (float)(((double)v[t + pxy] - (double)v0) * iz) : 0.f);
+  const unsigned pxy = (unsigned)(nx + 2) * (unsigned)(ny + 2);
+  const unsigned long long n = (unsigned long long)pxy * (nz + 2);
+  for (unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; t < n;
+       t += gridDim.x * (unsigned long long)blockDim.x) {
+    const unsigned k = (unsigned)t / pxy;  // padded layer
+    const float2 iz = k <= (unsigned)nz ? __ldg(iwz + k) : make_float2(0.f, 0.f);
+    const float v0 = __ldg(v + t);
+    float s = 0.f;
+    if (iz.x != 0.f) {
+      const float v1 = __ldg(v + t + pxy);
+      s = ff_mul(ff_diff(v1, v0), {iz.x, iz.y}).hi;
+      const float size = fabsf(v0) + fabsf(v1);
+      if (!(size == 0.f || (size > 1e-20f && size < 1e30f && fabsf(s) < 1e30f)))
+        s = (float)(((double)v1 - (double)v0) * ((double)iz.x + iz.y));
+    }
+    pairs[t] = make_float2(v0, s);
   }
 }
 
-// Negative-value flags (CubeDev::negflag) from the padded scalar grid: node
-// (i, j, k) is flagged when a node of [i-1, i+2] x [j-1, j+2] x [k-1, k+2],
-// clamped to the grid, is below zero.
+// Negative-value flags (CubeDev::negflag, zeroed before) from the padded
+// scalar grid: node (i, j, k) is flagged when a node of [i-1, i+2] x [j-1,
+// j+2] x [k-1, k+2], clamped to the grid, is below zero; each negative node
+// (few, as a rule) flags the up to 64 nodes whose block holds it.
 __global__ void cube_negflag_kernel(const float* __restrict__ v, int nx, int ny, int nz, uint8_t* __restrict__ flag) {
   const long long px = nx + 2, pxy = (long long)(nx + 2) * (ny + 2);
   const long long n = (long long)nx * ny * nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t % nx), j = (int)((t / nx) % ny), k = (int)(t / ((long long)nx * ny));
-    bool neg = false;
-    for (int kk = max(k - 1, 0); kk <= min(k + 2, nz - 1); ++kk)
-      for (int jj = max(j - 1, 0); jj <= min(j + 2, ny - 1); ++jj)
-        for (int ii = max(i - 1, 0); ii <= min(i + 2, nx - 1); ++ii)
-          neg |= v[(kk + 1) * pxy + (jj + 1) * px + (ii + 1)] < 0.f;
-    flag[t] = neg ? 1 : 0;
+    const unsigned row = (unsigned)t / (unsigned)nx;
+    const int i = (int)((unsigned)t - row * (unsigned)nx), k = (int)(row / (unsigned)ny), j = (int)(row - (unsigned)k * (unsigned)ny);
+    if (!(v[(k + 1) * pxy + (j + 1) * px + (i + 1)] < 0.f)) continue;
+    for (int kk = max(k - 2, 0); kk <= min(k + 1, nz - 1); ++kk)
+      for (int jj = max(j - 2, 0); jj <= min(j + 1, ny - 1); ++jj)
+        for (int ii = max(i - 2, 0); ii <= min(i + 1, nx - 1); ++ii) flag[((long long)kk * ny + jj) * nx + ii] = 1;
   }
 }
 
@@ -2491,13 +2587,13 @@ bool read_bounds_status(unsigned long long* status, bool reset) {
 #endif
 }
 
-cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, cudaStream_t s) {
+cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, int* neg, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int blocks = (int)std::min<long long>((n + 255) / 256, (long long)std::max(sms, 1) * 8);
-  cube_pad_copy_kernel<<<blocks, 256, 0, s>>>(src, nx, ny, nz, dst);
+  const int blocks = (int)std::min<long long>((n + 1023) / 1024, (long long)std::max(sms, 1) * 8);
+  cube_pad_copy_kernel<<<blocks, 256, 0, s>>>(src, (unsigned)n, nx, ny, nz, dst, neg);
   return cudaGetLastError();
 }
 
@@ -2511,23 +2607,25 @@ cudaError_t launch_cube_fill(const float*, int nx, int ny, int nz, float* dst, c
 cudaError_t launch_cube_negflags(const float* padded, int nx, int ny, int nz, uint8_t* flags, cudaStream_t s) {
   const long long n = (long long)nx * ny * nz;
   int blocks = (int)std::min<long long>((n + 255) / 256, 8192);
+  const cudaError_t e = cudaMemsetAsync(flags, 0, (size_t)n, s);
+  if (e != cudaSuccess) return e;
   cube_negflag_kernel<<<blocks, 256, 0, s>>>(padded, nx, ny, nz, flags);
   return cudaGetLastError();
 }
 
-cudaError_t launch_cube_records(const float* padded, int nx, int ny, int nz, const double* cx64, const double* cy64,
-                                const double* cz64, float4* rec, cudaStream_t s) {
+cudaError_t launch_cube_records(const float* padded, int nx, int ny, int nz, const float2* iwx, const float2* iwy,
+                                const float2* iwz, float4* rec, cudaStream_t s) {
   const long long n = (long long)(nx + 1) * (ny + 1) * (nz + 1);
   int blocks = (int)std::min<long long>((n + 255) / 256, 8192);
-  cube_records_kernel<<<blocks, 256, 0, s>>>(padded, nx, ny, nz, cx64, cy64, cz64, rec);
+  cube_records_kernel<<<blocks, 256, 0, s>>>(padded, nx, ny, nz, iwx, iwy, iwz, rec);
   return cudaGetLastError();
 }
 
-cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const double* cz64, float2* pairs,
+cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const float2* iwz, float2* pairs,
                               cudaStream_t s) {
   const long long n = (long long)(nx + 2) * (ny + 2) * (nz + 2);
   int blocks = (int)std::min<long long>((n + 255) / 256, 8192);
-  cube_pairs_kernel<<<blocks, 256, 0, s>>>(padded, nx, ny, nz, cz64, pairs);
+  cube_pairs_kernel<<<blocks, 256, 0, s>>>(padded, nx, ny, nz, iwz, pairs);
   return cudaGetLastError();
 }
 
