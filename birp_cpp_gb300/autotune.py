@@ -8,7 +8,8 @@ launch), over
     tiles up to 32 pixels a side;
       - for a request rendered alone (plain renders of the 256^3 stretched
         cube and of the default CMEM model from orbit poses), per
-        image-size and sample-count class, cube and CMEM requests apart;
+        image-size and sample-count class (each half the next), trilinear,
+        nearest and CMEM requests apart;
       - for a request inside a batch: 32-request batches of one class for
         trilinear and nearest cube requests, a 16-request batch of mixed
         sizes for CMEM requests;
@@ -39,6 +40,10 @@ ROOT = os.path.dirname(HERE)
 
 SIZES = [(144, 84), (288, 168), (576, 336), (1024, 600)]
 SAMPLES = [440, 880, 1760]
+# a request alone: its pixels decide how many lanes a ray gets to fill the
+# GPU once, so its classes are closer together
+PLAIN_SIZES = [(72, 42), (102, 60), (144, 84), (204, 119), (288, 168), (408, 238), (576, 336), (815, 475), (1024, 600)]
+PLAIN_SAMPLES = [110, 220, 440, 880, 1760]
 SEGMENTS = [1, 2, 4, 8]
 MAX_TILE = 32
 
@@ -62,7 +67,7 @@ def _timer(B, kind):
     import ctypes as C
     import torch  # device memory for the timed renders' output
     from birp_cpp_gb300 import synth
-    if kind == "cube":
+    if kind != "cmem":
         xs, ys, zs, v = synth.cube_config1(seed=1)
         space = B.Cube(xs, ys, zs, v.astype(np.float32))
         src = (space.h, None)
@@ -73,31 +78,35 @@ def _timer(B, kind):
     L = B.lib()
 
     def time_plain(cam, repeats):
-        ms = C.c_float()
-        B.check(L.birp_time_render_device(src[0], src[1], C.byref(cam), C.c_void_p(out.data_ptr()), repeats, 1,
-                                          C.byref(ms)))
-        return ms.value
+        """ms with a cold L2 plus ms with a warm one (a first and a repeated render)."""
+        total = 0.0
+        for flush in (1, 0):
+            ms = C.c_float()
+            B.check(L.birp_time_render_device(src[0], src[1], C.byref(cam), C.c_void_p(out.data_ptr()), repeats, flush,
+                                              C.byref(ms)))
+            total += ms.value
+        return total
 
     return space, time_plain
 
 
-def tune_plain(n_poses: int = 4, repeats: int = 3, kind: str = "cube"):
+def tune_plain(n_poses: int = 4, repeats: int = 5, kind: str = "tri"):
     """{(pixels, samples): (best (S, wx, gx), times)} for plain renders of
-    the 256^3 cube (kind "cube") or the default CMEM model ("cmem")."""
+    the 256^3 cube (kind "tri" or "nearest") or the default CMEM model ("cmem")."""
     import birp_cpp_gb300 as B
     from birp_cpp_gb300 import synth
     _space, time_plain = _timer(B, kind)
     poses = [(p, a) for p, a, *_ in synth.config2_requests(n_poses, seed=77)]
     results = {}
-    for nx, ny in SIZES:
-        for n in SAMPLES:
+    for nx, ny in PLAIN_SIZES:
+        for n in PLAIN_SAMPLES:
             times = {}
             for s in SEGMENTS:
                 for wx, gx in shapes(s):
                     tot = 0.0
                     for pos, aim in poses:
                         cam = B.camera(pos, aim, synth.FOV_W, synth.FOV_H, nx, ny, n_samples=n, segments=s,
-                                       warp_rays_x=wx, tile_warps_x=gx)
+                                       warp_rays_x=wx, tile_warps_x=gx, trilinear=kind != "nearest")
                         tot += time_plain(cam, repeats)
                     times[(s, wx, gx)] = tot / len(poses)
             best = min(times, key=times.get)
@@ -191,22 +200,25 @@ def _rows(results, kind_code=-1, trilinear=-1, all_sizes=False):
             if all_sizes:
                 nmax = 1 << 30
             s, wx, gx = results[(p, n)][0]
+            if j + 1 < len(smp) and results[(p, smp[j + 1])][0] == (s, wx, gx):
+                continue  # the next class's row covers this one
             out.append(f"    {{(int64_t){pmax}, {nmax}, {kind_code}, {trilinear}, {int(np.log2(s))}, "
                        f"{int(np.log2(wx))}, {int(np.log2(gx))}}},")
     return out
 
 
-def write_table(plain, plain_cmem, batch_tri, batch_near, batch_cmem, path):
+def write_table(plain, plain_near, plain_cmem, batch_tri, batch_near, batch_cmem, path):
     lines = ["// Tile-shape tables: the first row whose bounds hold gives the shape.",
              "// Columns: max pixels, max samples, kind (0 cube, 1 CMEM, -1 any), trilinear",
              "// (-1 any), log2(lanes per ray), log2(rays across a warp block), log2(warps",
              "// across a tile) (-1: the default for the lanes per ray). Written by",
              "// birp_cpp_gb300/autotune.py from timings on a GB300 (256^3 stretched cube or",
-             "// the default CMEM model, orbit poses, L2 flushed before each launch): plain",
-             "// renders for a request alone (CMEM and cube requests), 32-request batches of",
-             "// one cube class and a 16-request mixed-size CMEM batch for a request inside",
-             "// a batch.",
-             "static const TuneRow kTuneRowsPlain[] = {"] + _rows(plain_cmem, 1, -1) + _rows(plain) + ["};",
+             "// the default CMEM model, orbit poses): plain renders for a request alone (with",
+             "// a cold and with a warm L2; CMEM, nearest and trilinear requests), 32-request",
+             "// batches of one cube class and a 16-request mixed-size CMEM batch for a",
+             "// request inside a batch (with a cold L2).",
+             "static const TuneRow kTuneRowsPlain[] = {"] + _rows(plain_cmem, 1, -1) + _rows(plain_near, 0, 0) + \
+            _rows(plain) + ["};",
              "static const TuneRow kTuneRowsBatch[] = {"] + _rows(batch_cmem, 1, -1, all_sizes=True) + \
             _rows(batch_near, 0, 0) + _rows(batch_tri, -1, -1) + ["};"]
     with open(path, "w") as f:
@@ -317,11 +329,12 @@ def main():
         build.build()
         B.init(0)
         plain = tune_plain(args.poses, args.repeats)
+        plain_near = tune_plain(args.poses, args.repeats, kind="nearest")
         plain_cmem = tune_plain(args.poses, args.repeats, kind="cmem")
         tri = tune_batch("tri", repeats=args.repeats)
         near = tune_batch("nearest", repeats=args.repeats)
         cm = tune_batch_cmem(repeats=args.repeats)
-        write_table(plain, plain_cmem, tri, near, cm, args.out)
+        write_table(plain, plain_near, plain_cmem, tri, near, cm, args.out)
         print("wrote", args.out)
 
 
