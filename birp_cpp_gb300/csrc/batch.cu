@@ -78,9 +78,9 @@ birp_status batch_create(int max_requests, int64_t max_pixels, birp_batch** out)
   cudaError_t e;
   if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaHostAlloc(&b->h_stage, b->stage_bytes, cudaHostAllocDefault)) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_stage, b->stage_bytes)) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_counter, BATCH_CLASSES * sizeof(unsigned int))) != cudaSuccess ||
-      (e = cudaMalloc(&b->d_out, (size_t)max_pixels * sizeof(float))) != cudaSuccess ||
+      (e = device_alloc((void**)&b->d_stage, b->stage_bytes)) != cudaSuccess ||
+      (e = device_alloc((void**)&b->d_counter, BATCH_CLASSES * sizeof(unsigned int))) != cudaSuccess ||
+      (e = device_alloc((void**)&b->d_out, (size_t)max_pixels * sizeof(float))) != cudaSuccess ||
       (e = cudaHostAlloc(&b->h_out, (size_t)max_pixels * sizeof(float), cudaHostAllocDefault)) != cudaSuccess ||
       (e = cudaEventCreate(&b->e_start)) != cudaSuccess || (e = cudaEventCreate(&b->e_kernel)) != cudaSuccess ||
       (e = cudaEventCreate(&b->e_end)) != cudaSuccess ||

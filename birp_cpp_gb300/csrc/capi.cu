@@ -263,7 +263,7 @@ birp_status ensure_scratch(size_t img_floats) {
   g.scratch = nullptr;
   g.scratch_floats = 0;
   size_t want = std::max(img_floats, (size_t)1 << 20);
-  cudaError_t e = cudaMalloc(&g.scratch, want * sizeof(float));
+  cudaError_t e = device_alloc((void**)&g.scratch, want * sizeof(float));
   if (e != cudaSuccess) return fail(BIRP_ERR_NOMEM, "cudaMalloc(%zu B) for the image: %s", want * 4, cudaGetErrorString(e));
   g.scratch_floats = want;
   return BIRP_OK;
@@ -376,6 +376,7 @@ void birp_shutdown(void) {
   if (g_ctx.device < 0) return;
   cudaSetDevice(g_ctx.device);
   cudaStreamSynchronize(g_ctx.stream);
+  block_release_all();
   if (g_ctx.scratch) cudaFree(g_ctx.scratch);
   if (g_ctx.flush) cudaFree(g_ctx.flush);
   if (g_ctx.stats) cudaFree(g_ctx.stats);
@@ -521,7 +522,7 @@ birp_status birp_cmem_create(const birp_cmem_params* p, birp_cmem** out) {
   cmem_coefficients(*p, m->h_desc);
   // one allocation: the descriptor, then its table of surface bounds
   constexpr size_t table_off = (sizeof(CmemDev) + 255) / 256 * 256;
-  cudaError_t e = cudaMalloc(&m->d_desc, table_off + sizeof(float4) * kCmemCt * kCmemCp);
+  cudaError_t e = device_alloc((void**)&m->d_desc, table_off + sizeof(float4) * kCmemCt * kCmemCp);
   if (e != cudaSuccess) {
     delete m;
     return fail(BIRP_ERR_NOMEM, "cudaMalloc: %s", cudaGetErrorString(e));

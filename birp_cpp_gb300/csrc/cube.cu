@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "birp_host.h"
@@ -92,10 +93,73 @@ birp_status ensure_xyz_scratch(size_t floats) {
   g.xyz_scratch = nullptr;
   g.xyz_floats = 0;
   size_t want = std::max(floats, (size_t)1 << 16);
-  cudaError_t e = cudaMalloc(&g.xyz_scratch, want * sizeof(float));
+  cudaError_t e = device_alloc((void**)&g.xyz_scratch, want * sizeof(float));
   if (e != cudaSuccess) return fail(BIRP_ERR_NOMEM, "cudaMalloc: %s", cudaGetErrorString(e));
   g.xyz_floats = want;
   return BIRP_OK;
+}
+
+namespace {
+struct Block {
+  void* p;
+  size_t bytes;
+};
+std::mutex g_blocks_mu;
+std::vector<Block> g_blocks;  // kept blocks, oldest first
+size_t g_blocks_bytes = 0;
+constexpr size_t kKeepMin = (size_t)8 << 20, kKeepMax = (size_t)1 << 30;
+}  // namespace
+
+void block_release_all() {
+  std::lock_guard<std::mutex> lk(g_blocks_mu);
+  for (const Block& b : g_blocks) cudaFree(b.p);
+  g_blocks.clear();
+  g_blocks_bytes = 0;
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    block_release_all();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
+cudaError_t block_alloc(void** p, size_t* bytes) {
+  if (*bytes >= kKeepMin) {
+    std::lock_guard<std::mutex> lk(g_blocks_mu);
+    size_t best = g_blocks.size();
+    for (size_t i = 0; i < g_blocks.size(); ++i)  // the smallest that fits, at most an eighth larger
+      if (g_blocks[i].bytes >= *bytes && g_blocks[i].bytes <= *bytes + *bytes / 8 &&
+          (best == g_blocks.size() || g_blocks[i].bytes < g_blocks[best].bytes))
+        best = i;
+    if (best < g_blocks.size()) {
+      *p = g_blocks[best].p;
+      *bytes = g_blocks[best].bytes;
+      g_blocks_bytes -= g_blocks[best].bytes;
+      g_blocks.erase(g_blocks.begin() + (long)best);
+      return cudaSuccess;
+    }
+  }
+  return device_alloc(p, *bytes);
+}
+
+void block_free(void* p, size_t bytes, bool device_idle) {
+  if (!p) return;
+  if (bytes < kKeepMin || bytes > kKeepMax || !device_idle || g_ctx.device < 0) {
+    cudaFree(p);
+    return;
+  }
+  std::lock_guard<std::mutex> lk(g_blocks_mu);
+  while (!g_blocks.empty() && g_blocks_bytes + bytes > kKeepMax) {
+    cudaFree(g_blocks.front().p);
+    g_blocks_bytes -= g_blocks.front().bytes;
+    g_blocks.erase(g_blocks.begin());
+  }
+  g_blocks.push_back({p, bytes});
+  g_blocks_bytes += bytes;
 }
 
 void destroy_cube_device(birp_cube& c) {
@@ -105,8 +169,13 @@ void destroy_cube_device(birp_cube& c) {
                     (void*)c.d_grid, (void*)c.d_pairs, (void*)c.d_walk4, (void*)c.d_nodes_ff, (void*)c.d_negflag})
       if (p) cudaFreeAsync(p, c.alloc_stream);
   } else {
-    for (void* p : {(void*)c.d_vals, (void*)c.d_c64, (void*)c.d_lut, (void*)c.d_desc, (void*)c.d_cells,
-                    (void*)c.d_grid, (void*)c.d_pairs, (void*)c.d_walk4, (void*)c.d_nodes_ff, (void*)c.d_negflag})
+    // a freed block waits for the device, and so does one that is kept
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    block_free(c.d_vals, c.vals_bytes, idle);
+    block_free(c.d_grid, c.grid_bytes, idle);
+    block_free(c.d_pairs, c.pairs_bytes, idle);
+    for (void* p : {(void*)c.d_c64, (void*)c.d_lut, (void*)c.d_desc, (void*)c.d_cells, (void*)c.d_walk4,
+                    (void*)c.d_nodes_ff, (void*)c.d_negflag})
       if (p) cudaFree(p);
   }
   c.d_pairs = nullptr;
@@ -131,7 +200,20 @@ void destroy_cube_device(birp_cube& c) {
 
 template <class T>
 static cudaError_t dev_alloc(T** p, size_t bytes, cudaStream_t alloc_stream) {
-  return alloc_stream ? cudaMallocAsync((void**)p, bytes, alloc_stream) : cudaMalloc((void**)p, bytes);
+  if (!alloc_stream) return device_alloc((void**)p, bytes);
+  cudaError_t e = cudaMallocAsync((void**)p, bytes, alloc_stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    block_release_all();
+    e = cudaMallocAsync((void**)p, bytes, alloc_stream);
+  }
+  return e;
+}
+// a large array: from the kept blocks outside a server
+template <class T>
+static cudaError_t big_alloc(T** p, size_t* held, size_t bytes, cudaStream_t alloc_stream) {
+  *held = bytes;
+  return alloc_stream ? dev_alloc(p, bytes, alloc_stream) : block_alloc((void**)p, held);
 }
 
 birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool stream_alloc) {
@@ -221,16 +303,16 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
       }
   }
   const size_t iw_off = (total * sizeof(float) + 7) / 8 * 8, neg_off = iw_off + iw.size() * sizeof(float2);
-  CKU(dev_alloc(&scalar, neg_off + (find_neg ? sizeof(int) : 0), c.alloc_stream));
+  CKU(big_alloc(&scalar, &c.grid_bytes, neg_off + (find_neg ? sizeof(int) : 0), c.alloc_stream));
   float2* const d_iw = reinterpret_cast<float2*>(reinterpret_cast<char*>(scalar) + iw_off);
   int* const d_neg = find_neg ? reinterpret_cast<int*>(reinterpret_cast<char*>(scalar) + neg_off) : nullptr;
   c.d_grid = scalar;
   if (nodes_layout) {
     CKU(dev_alloc(&c.d_walk4, walk.size() * sizeof(float4), c.alloc_stream));
-    if (pairs) CKU(dev_alloc(&c.d_pairs, total * sizeof(float2), c.alloc_stream));
+    if (pairs) CKU(big_alloc(&c.d_pairs, &c.pairs_bytes, total * sizeof(float2), c.alloc_stream));
   } else {
     CKU(dev_alloc(&c.d_cells, walk2.size() * sizeof(float2), c.alloc_stream));
-    CKU(dev_alloc(&c.d_vals, records * 2 * sizeof(float4), c.alloc_stream));
+    CKU(big_alloc(&c.d_vals, &c.vals_bytes, records * 2 * sizeof(float4), c.alloc_stream));
     // the walk reads a record with one 32-byte load, which needs 32-byte
     // alignment (device allocations are 256-byte aligned)
     if (reinterpret_cast<uintptr_t>(c.d_vals) % 32 != 0)
@@ -371,7 +453,7 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   CKU(cudaStreamSynchronize(st));
   if (!compact && !c.alloc_stream) {
     c.d_grid = nullptr;
-    CKU(cudaFree(scalar));
+    block_free(scalar, c.grid_bytes, true);  // the stream that used it is done
   }
   return BIRP_OK;
 }
