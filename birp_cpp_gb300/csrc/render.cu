@@ -53,9 +53,9 @@ constexpr int kThreads = 128;
 #define BIRP_CMEM_MINB BIRP_CMEM_MINB_TUNED  // CMEM
 #endif
 #ifndef BIRP_SIGNED_MINB
-// trilinear cubes holding negative values (any layout; at 5 or 6 CTAs per SM
-// the float-float cell function spills: 12 orbit renders 2.21 -> 4.13 / 5.12 ms)
-#define BIRP_SIGNED_MINB 4
+// trilinear cubes holding negative values (any layout; 12 views, mean of 12 sets,
+// at 5, 6, 7 and 8 CTAs per SM: 1.59, 1.56, 1.61, 1.64 ms)
+#define BIRP_SIGNED_MINB 6
 #endif
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
@@ -146,6 +146,12 @@ __device__ __forceinline__ FF ff_mul(FF x, FF y) {
   const float e = fmaf(x.hi, y.lo, fmaf(x.lo, y.hi, fmaf(x.hi, y.hi, -p)));
   return ff_quick(p, e);
 }
+__device__ __forceinline__ FF ff_diff(float a, float b) {  // a - b, exactly
+  FF r;
+  two_sum(a, -b, r.hi, r.lo);
+  return r;
+}
+__device__ __forceinline__ FF ff_sub(FF a, FF b) { return ff_add(a, {-b.hi, -b.lo}); }
 // 1/x: one Newton step r + r (1 - x r) from the FP32 reciprocal
 __device__ __forceinline__ FF ff_recip(FF x) {
   const float r = 1.f / x.hi;
@@ -772,11 +778,10 @@ struct LaneRun {
 // of their rate). A sample's cell and sign are decided within the stated
 // bounds of that arithmetic, which cover the oracle's own FP64 rounding; what
 // they leave open (and corners that are not finite) takes the oracle's FP64.
-// Bound by the rays that enter such cells (latency: 16 warps per SM, the
-// function's registers). 12 orbit renders of a 192x160x176 cube with 1e-5 of
-// its nodes negative: 16.5 ms with a scan of every sample before the walk and
-// FP64 signs and sums, 2.21 ms so.
-// (g0..g2: the walk's cell, a guess.) Not inlined: it runs only in such cells.
+// 12 orbit renders of a 192x160x176 cube with 1e-5 of its nodes negative (mean
+// over 12 sets): 16.5 ms with a scan of every sample before the walk and FP64
+// signs and sums, 2.29 ms with this function sample by sample, 2.12 ms with
+// whole cells by the closed form, 1.56 ms called for all held lanes at once.
 __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* a, const double* b, int i0, int i1,
                                             int g0, int g1, int g2, LaneRun run, int first, float2* sum) {
   const RequestDev& R = *Rp;
@@ -799,6 +804,65 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
     bs[r] = ff_add({R.pos_hi[r], R.pos_lo[r]}, {0.5f * st[r].hi, 0.5f * st[r].lo});
     e[r] = 2e-13f * (fabsf(R.pos32[r]) + (float)R.N * R.dt32 + fmaxf(fabsf((float)A.c_first), fabsf((float)A.c_last)));
     k[r] = min(max(k[r], 0), A.n - 2);
+  }
+  auto lerp = [](FF p, FF q, FF t) { return ff_add(p, ff_mul(ff_sub(q, p), t)); };
+  // The walk's cell holds every sample when the first and the last lie in it by
+  // more than e. Then corners that are all good (most flagged cells: only a
+  // neighbour's are negative) make every sample good, and the samples' sum is
+  // the closed form of the march (about their middle), in float-float; and
+  // negative corners make every sample negative.
+  {
+    bool inside = true;
+    FF f[3], step[3];
+    const float mid = 0.5f * (float)(i0 + i1 - 1), m = (float)(i1 - i0);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const float2 c0 = __ldg(C.nodes_ff[r] + k[r]), c1 = __ldg(C.nodes_ff[r] + k[r] + 1);
+      for (int last = 0; last < 2; ++last) {
+        const FF x = ff_add(bs[r], ff_mul(st[r], {(float)(last ? i1 - 1 : i0), 0.f}));
+        inside = inside && (x.hi - c0.x) + (x.lo - c0.y) > e[r] && (c1.x - x.hi) + (c1.y - x.lo) > e[r];
+      }
+      const FF iw = ff_recip(ff_sub({c1.x, c1.y}, {c0.x, c0.y}));
+      f[r] = ff_mul(ff_sub(ff_add(bs[r], ff_mul(st[r], {mid, 0.f})), {c0.x, c0.y}), iw);
+      step[r] = ff_mul(st[r], iw);
+    }
+    float v[8], mn = INFINITY, mx = -INFINITY, size = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      v[q] = node_value(C, k[0] + (q & 1), k[1] + ((q >> 1) & 1), k[2] + (q >> 2));
+      mn = fminf(mn, v[q]);
+      mx = fmaxf(mx, v[q]);
+      size += fabsf(v[q]);
+    }
+    // (with room for the low parts: else one by one)
+    const bool fits = size == 0.f || (size > 1e-20f && size < 1e30f);
+    if (inside && fits && mx < 0.f) {
+      if (i0 == first) run.first_neg = true;
+      if (run.phase == RUN_GOOD) run.phase = RUN_ENDED;
+      return run;
+    }
+    if (inside && fits && mn >= 0.f) {
+      FF ex[4];  // differences along x of the four edges
+#pragma unroll
+      for (int q = 0; q < 4; ++q) ex[q] = ff_diff(v[2 * q + 1], v[2 * q]);
+      FF y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = ff_add({v[2 * q], 0.f}, ff_mul(ex[q], f[0]));
+      const FF z0 = lerp(y[0], y[1], f[1]), z1 = lerp(y[2], y[3], f[1]);
+      const FF value = lerp(z0, z1, f[2]);
+      const FF fxy = lerp(ff_sub(ex[1], ex[0]), ff_sub(ex[3], ex[2]), f[2]);
+      const FF fxz = lerp(ff_sub(ex[2], ex[0]), ff_sub(ex[3], ex[1]), f[1]);
+      const FF fyz = ff_sub(ff_sub(y[3], y[2]), ff_sub(y[1], y[0]));
+      const FF p2 = ff_add(ff_add(ff_mul(fxy, ff_mul(step[0], step[1])), ff_mul(fxz, ff_mul(step[0], step[2]))),
+                           ff_mul(fyz, ff_mul(step[1], step[2])));
+      // sum of (i - mid)^2 / m = (m^2 - 1) / 12
+      const FF spread = ff_mul(ff_sub(ff_mul({m, 0.f}, {m, 0.f}), {1.f, 0.f}), ff_recip({12.f, 0.f}));
+      const FF total = ff_mul({m, 0.f}, ff_add(value, ff_mul(p2, spread)));
+      run.phase = RUN_GOOD;
+      run.n += i1 - i0;
+      *sum = make_float2(total.hi, total.lo);
+      return run;
+    }
   }
   FF s = {sum->x, sum->y};
   for (int i = i0; i < i1 && run.phase != RUN_ENDED; ++i) {
@@ -840,7 +904,6 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
       if (mx < 0.f) {
         neg = true;  // every interpolation of negative corners is
       } else {
-        auto lerp = [](FF p, FF q, FF t) { return ff_add(p, ff_mul(ff_add(q, {-p.hi, -p.lo}), t)); };
         auto lerp1 = [](float p, float q, FF t) {
           float d, r;
           two_sum(q, -p, d, r);
@@ -1251,8 +1314,36 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
     const float4* q = C.rec;
     [[maybe_unused]] const float* g = C.grid;
     [[maybe_unused]] const float2* gp = reinterpret_cast<const float2*>(C.grid);
-    if (count > 0) {
-      const float f0 = (float)first_c;
+    // SIGNED: the warp's lanes walk until each is done or held in a flagged
+    // cell (an iteration leaves a held lane as it is); signed_cell then looks
+    // at the held lanes' cells, all in one call, and each sets out again from
+    // its next sample. With a call inside the walk, lane by lane, the walk's
+    // registers were reloaded from the stack by every cell and the class held
+    // to 4 CTAs per SM (mean of 12 views of a cube with 1e-5 of its nodes
+    // negative 2.12 -> 1.56 ms; stopping at the first held lane 2.22, at 8 held
+    // 1.88, at 16 1.74). Others walk once.
+    int at = first_c, left = count;  // the part of the run still to walk
+    float ncell = 0.f;               // cells summed: at most 2^22, exact
+    for (;;) {
+    [[maybe_unused]] bool flagged = false;
+    [[maybe_unused]] int fi = 0, fs[3] = {0, 0, 0};  // the cell's flag, its steps per axis
+    float u = 0.f, nxt = 0.f;
+    [[maybe_unused]] unsigned walkers = 0;
+    if constexpr (SIGNED) {
+      walkers = __ballot_sync(0xffffffffu, left > 0);
+      if (walkers == 0) break;
+      asm volatile("" ::: "memory");  // the set-up below is done again, not kept
+      float w[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) w[k] = (float)__dadd_rn(sm.A[lx][k], sm.B[ly][k]);
+      const float inv = rsqrtf(fmaf(w[0], w[0], fmaf(w[1], w[1], w[2] * w[2])));
+#pragma unroll
+      for (int k = 0; k < 3; ++k) d32[k] = w[k] * inv;
+      g = C.grid;
+      gp = reinterpret_cast<const float2*>(C.grid);
+    }
+    if (left > 0) {
+      const float f0 = (float)at;
       int k0s[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
@@ -1299,11 +1390,16 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
       const float hx = 0.5f * st[0], hy = 0.5f * st[1], hz = 0.5f * st[2];
       const float Dxy = st[0] * st[1] * (1.f / 12.f), Dxz = st[0] * st[2] * (1.f / 12.f),
                   Dyz = st[1] * st[2] * (1.f / 12.f);
-      const float ub = (float)count;
-      float u = 0.f;
-      float ncell = 0.f;  // cells summed: at most 2^22, exact
-      [[maybe_unused]] int cj[3] = {k0s[0], k0s[1], k0s[2]};
+      const float ub = (float)left;
+      if constexpr (SIGNED) {
+        const int fy = C.ax[0].n, fz = fy * C.ax[1].n;
+        fi = k0s[2] * fz + k0s[1] * fy + k0s[0];
+        fs[0] = signbit(d32[0]) ? -1 : 1;
+        fs[1] = signbit(d32[1]) ? -fy : fy;
+        fs[2] = signbit(d32[2]) ? -fz : fz;
+      }
       [[maybe_unused]] bool all_exact = false;
+      [[maybe_unused]] const unsigned flags_end = SIGNED ? (unsigned)C.neg_n - 1u : 0u;
       if constexpr (SIGNED) {
         // bound on |FP32 cell index - exact index|: position error (step,
         // position and coordinate roundings) over the smallest cell, the
@@ -1313,7 +1409,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
                                      C.neg_cmax) + 1e-6f;
         all_exact = fmaf(e_pos, C.neg_inv_gap, 2e-6f * (float)C.neg_nmax + 1e-6f) >= 1.f;
       }
-      while (u < ub) {
+      while (SIGNED || u < ub) {
         float4 lo, hi;  // {c0, c3, c1, c5}, {c2, c6, c4, c7}
         if constexpr (COMPACT) {
           // the cell's trilinear coefficients from its 8 corners, in local
@@ -1360,36 +1456,18 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         }
         // the first sample past the cell; not behind u, where a plane passed
         // before sample u is still to be stepped (such a cell holds no sample)
-        const float nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
+        nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
         // a cube holding negative values: the samples of a cell next to a
-        // negative node (its flag) are looked at one by one; an unflagged
-        // cell's are all good, as its FP32 cell is within one of the exact
-        // one (unless all_exact)
-        bool exact_cell_sum = false;
+        // negative node are looked at by signed_cell; an unflagged cell's are
+        // all good, as its FP32 cell is within one of the exact one (unless
+        // all_exact). So are those of a guard cell (the only ones with an
+        // infinite exit plane), which has no flag.
         if constexpr (SIGNED) {
-          if (nxt > u) {
-            const int cx = min(max(cj[0], 0), C.ax[0].n - 2), cy = min(max(cj[1], 0), C.ax[1].n - 2),
-                      cz = min(max(cj[2], 0), C.ax[2].n - 2);
-            long long fi = ((long long)cz * C.ax[1].n + cy) * C.ax[0].n + cx;
-#ifdef BIRP_DEBUG_BOUNDS
-            if (!bound_ok(fi, C.neg_n, 3)) fi = 0;
-#endif
-            if (all_exact || __ldg(C.negflag + fi)) {
-              float2 s2 = make_float2(0.f, 0.f);
-              run = signed_cell(&R, sm.A[lx], sm.B[ly], first_c + (int)u, first_c + (int)nxt, cx, cy, cz, run, first_c,
-                                &s2);
-              acc.add(s2.x);
-              acc.add(s2.y);
-              u = run.phase == RUN_ENDED ? ub : nxt;  // (no break: the lanes would not meet again)
-              ncell += 1.f;
-              exact_cell_sum = true;
-            } else {
-              run.phase = RUN_GOOD;
-              run.n += (int)(nxt - u);
-            }
-          }
+          const unsigned fc = min((unsigned)fi, flags_end);
+          flagged = nxt > u && (all_exact || __ldg(C.negflag + fc) || fmaxf(fmaxf(ex[0], ex[1]), ex[2]) == INFINITY);
+          if (!__any_sync(walkers, u < ub && !flagged)) break;
         }
-        if (!exact_cell_sum) {
+        {
           // The cell's m samples, u .. nxt - 1, lie symmetrically about their
           // middle c = (u + nxt - 1) / 2, so the odd powers of the cubic
           // about c drop out of their sum: m f(c) + p2 sum (i - c)^2 =
@@ -1449,10 +1527,10 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
           // a cell without a sample (rare: two planes of one axis between two
           // samples) goes through the same instructions with weight 0, and
           // its value, which may be an infinity, is not used
-          const bool any = nxt > u;
+          const bool any = nxt > u && !(SIGNED && flagged);
           acc.add_product(m, any ? mean : 0.f);
           ncell += any ? 1.f : 0.f;
-          u = nxt;
+          u = SIGNED && flagged ? u : nxt;
         }
         // step each axis whose exit index has been reached, once: a second
         // plane passed before the next sample is stepped in the next
@@ -1482,12 +1560,28 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
             } else {
               q += dstr[k];
             }
-            if constexpr (SIGNED) cj[k] += signbit(d32[k]) ? -1 : 1;
+            if constexpr (SIGNED) fi += fs[k];
           }
         }
       }
-      n_cells = (unsigned int)ncell;
     }
+    if constexpr (!SIGNED) break;
+    if (u > 0.f) run.phase = RUN_GOOD;  // the walk sums good samples only
+    run.n += (int)u;
+    if (flagged) {
+      float2 s2 = make_float2(0.f, 0.f);
+      const int row = fi / C.ax[0].n;
+      run = signed_cell(&R, sm.A[lx], sm.B[ly], at + (int)u, at + (int)nxt, fi - row * C.ax[0].n, row % C.ax[1].n,
+                        row / C.ax[1].n, run, first_c, &s2);
+      acc.add(s2.x);
+      acc.add(s2.y);
+      u = nxt;
+      ncell += 1.f;
+    }
+    at += (int)u;
+    left = run.phase == RUN_ENDED ? 0 : left - (int)u;
+    }
+    n_cells = (unsigned int)ncell;
   } else if constexpr (KIND == SPACE_CUBE) {
     // Nearest by truncation, walked cell by cell. A sample takes the value of
     // the lower node of the cell that holds it (DataCube::GetSample,
@@ -2087,13 +2181,6 @@ __device__ __noinline__ void cell_record64(const float* v, const double* i3, flo
   const double c[8] = {v000, c3, c1, c5, c2, c6, c4, c7};
   for (int k = 0; k < 8; ++k) out[k] = (float)c[k];
 }
-__device__ __forceinline__ FF ff_diff(float a, float b) {  // a - b, exactly
-  FF r;
-  two_sum(a, -b, r.hi, r.lo);
-  return r;
-}
-__device__ __forceinline__ FF ff_sub(FF a, FF b) { return ff_add(a, {-b.hi, -b.lo}); }
-
 // (bound by the store of the records: 13.8 M cells, 440 MB, 1.43 ms with FP64
 // arithmetic, 0.134 ms so, 3.7 TB/s read and written)
 __global__ void cube_records_kernel(const float* __restrict__ v, int nx, int ny, int nz, const float2* __restrict__ iwx,
