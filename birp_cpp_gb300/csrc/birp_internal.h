@@ -5,7 +5,7 @@
 //    trilinear polynomial f = c0 + c1 x + c2 y + c3 z + c4 xy + c5 xz + c6 yz
 //    + c7 xyz in the cell's local coordinates (x, y, z) = p - (lower node)
 //    (physical units, so a ray's step along an axis is the same in every
-//    cell), computed in FP64 from the FP32 corner values and stored FP32 as
+//    cell), computed in float-float from the FP32 corner values and stored FP32 as
 //    {c0, c3, c1, c5 | c2, c6, c4, c7} (the pairs the march's packed FP32x2
 //    FMAs take: {c0, c3}, {c1, c5}, {c2, c6}, {c4, c7}); c0 is the value of the cell's lower
 //    corner (node k). Records are x fastest for cells -1..n-1 on every axis:
@@ -27,7 +27,7 @@
 //  * pairs layout (the middle ground: about 2x the input, near the records
 //    layout's speed): the same padded grid, each node a float2 {v, s} of its
 //    value and the slope of its z-edge, s = (v(k+1) - v(k)) / (z(k+1) - z(k))
-//    computed in FP64 (0 on the guard cells along z), so a cell's 4 z-edges
+//    computed in float-float (0 on the guard cells along z), so a cell's 4 z-edges
 //    {c + s z} are 4 8-byte loads whose differences along x and y give its 8
 //    coefficients; float4 walk tables as in the compact layout.
 //  * per-axis index tables (LUT) for nonuniform axes: float4 bins of width at
@@ -154,7 +154,7 @@ struct RequestDev {
 // Status/counters the kernels report (device memory, read by the host).
 struct KernelStats {
   unsigned long long exact_range_rays;   // rays whose in-box range needed FP64
-  unsigned long long exact_nearest;      // nearest-mode samples decided in FP64
+  unsigned long long exact_nearest;      // nearest-mode samples of the runs summed in FP64
   unsigned long long exact_cmem;         // CMEM samples decided in FP64
   unsigned long long items;              // work items rendered (persistent kernel)
   unsigned long long samples;            // ray-samples evaluated

@@ -66,7 +66,7 @@ birp_status birp_cube_create(const double* xs, int nx, const double* ys, int ny,
  *            the FP32 values; the fastest to render (the default).
  *   PAIRS:   per node its FP32 value and the slope of its z-edge, plus a guard
  *            layer, about 2x; the kernels form a cell's coefficients from its
- *            4 z-edges (6 differences, 7 products). About 1.2x the records
+ *            4 z-edges (6 differences, 6 products). About 1.2x the records
  *            layout's render time at a quarter of its memory.
  *   COMPACT: the FP32 node values plus a guard layer, about 1x; the kernels
  *            form each cell's coefficients from its 8 corners. For holding
@@ -304,7 +304,7 @@ birp_status birp_server_get_stats(const birp_server* s, birp_server_stats* st);
 
 typedef struct {
   uint64_t exact_range_rays;   /* rays whose in-box range was decided in FP64 */
-  uint64_t exact_nearest;      /* nearest-mode samples decided in FP64 */
+  uint64_t exact_nearest;      /* nearest-mode samples of the runs summed in FP64 */
   uint64_t exact_cmem;         /* CMEM samples decided in FP64 */
   uint64_t items;              /* tiles rendered by the persistent kernel */
   uint64_t samples;            /* ray-samples evaluated (the roofline's unit) */
