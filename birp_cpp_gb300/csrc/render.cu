@@ -1706,38 +1706,49 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         ds[k] = up ? stride : -stride;  // in cells
         dn[k] = up ? 1 : -1;
       }
-      // The walk. Per axis ex is the FP32 crossing index of the next plane, one
-      // FMA a step; a crossing is looked at closely only when it is the next
-      // one and within E of an integer: then float-float (the pairs wait in
-      // shared memory), and within that bound the oracle's predicate, decide
-      // it, and ex becomes (first sample past the plane) - 1/2, certain from
-      // there on. An axis is stepped when its crossing lies before the current
-      // sample by more than E. An axis along which the ray hardly moves (E
-      // above 0.015; 0.005 to 0.03 within 4 %, 0.1 5 % and 0.002 29 % slower)
-      // gets no estimate, and so does not widen E for the others: its ex is
-      // far below any sample, so its plane is always decided closely, and
-      // first of all.
-      // Bound by issue and the close looks' chains (a warp has one in 1 of 8
-      // iterations). 24 orbit renders of the 256^3 cube, pairs layout: 3.97 ms
-      // with one certified crossing per iteration picked by selects, 3.2 ms
-      // so; records 4.12 -> 3.4 ms.
+      // The walk. Per axis ex is the crossing index of the next plane from the
+      // float pairs of P, 1 / (d dt) and K, the low parts' products summed apart
+      // and the sum left unnormalised: 4 FP32 operations for an error of
+      // 1.9e-7 (N + 2), where the high parts alone (one FMA) left up to 0.015. A
+      // crossing is looked at closely only when it is the next one and within
+      // E of an integer: then float-float (the pairs wait in shared memory),
+      // and within that bound the oracle's predicate, decide it, and ex becomes
+      // (first sample past the plane) - 1/2, certain from there on. An axis is
+      // stepped when its crossing lies before the current sample by more than
+      // E. An axis whose E is above 0.015 (a ray of tens of thousands of samples,
+      // or 1 / (d dt) beyond 1e9) gets no estimate, and so does not widen E for
+      // the others: its ex is far below any sample, so its plane is always
+      // decided closely, and first of all.
+      // Bound by the iteration's chain (load, 4 operations, minimum) and issue.
+      // 24 orbit renders of the 256^3 cube, pairs layout: 3.97 ms with one
+      // certified crossing per iteration picked by selects, 3.18 ms with the
+      // one-FMA estimate (a warp looked closely in 1 of 8 iterations, at 2 of
+      // its lanes), 2.86 ms so; records 4.12, 3.38, 3.07 ms.
       __shared__ float pairs[12][kThreads];
-      float ex[3], fi32[3], fK[3], E = 0.f;
+      float ex[3], fi32[3], fK[3], fil[3], fKl[3], E = 0.f;
       int ni[3];  // the next planes as indices into the node table of all three axes
       const float2* nbase = C.nodes_ff[0];
+      auto crossing = [&](int k, float2 P) -> float {  // NaN or inf at a sentinel: fminf and <= pass it over
+        return fmaf(P.x, fi32[k], -fK[k]) + fmaf(P.y, fi32[k], fmaf(P.x, fil[k], -fKl[k]));
+      };
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         pairs[4 * k][tid] = inv[k].hi;
         pairs[4 * k + 1][tid] = inv[k].lo;
         pairs[4 * k + 2][tid] = K[k].hi;
         pairs[4 * k + 3][tid] = K[k].lo;
-        const float Ek = fmaf(6.1e-8f, (float)(N + 2), E32[k]);  // and the rounding of u - E below
+        // `closely` below: u as in `cross` with its bound, the product of the
+        // low parts left out and the low terms' roundings (7 x 2^-48 cp |inv|),
+        // the two roundings of its sum (2^-24 |u| each) and that of u - E below
+        const float Ek = fmaf(6e-14f * cp[k], fabsf(inv[k].hi), fmaf(1.9e-7f, (float)(N + 2), 1e-8f));
         const bool good = Ek <= 0.015f;
         if (good) E = fmaxf(E, Ek);
         fi32[k] = good ? inv[k].hi : 0.f;
         fK[k] = good ? K[k].hi : 3e38f;
+        fil[k] = good ? inv[k].lo : 0.f;
+        fKl[k] = good ? K[k].lo : 0.f;
         ni[k] = (int)(np[k] - nbase);
-        ex[k] = w64[k] == 0.0 ? INFINITY : fmaf(__ldg(np[k]).x, fi32[k], -fK[k]);
+        ex[k] = w64[k] == 0.0 ? INFINITY : crossing(k, __ldg(np[k]));
       }
       // first sample past the plane of node index nk along axis k, in
       // float-float: INFINITY when no sample of the ray is
@@ -1821,7 +1832,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
 #ifdef BIRP_DEBUG_BOUNDS
             if (!bound_ok(nd - (C.nodes_ff[0] - 1), C.nodes_n, 8)) nd = C.nodes_ff[0];
 #endif
-            ex[k] = fmaf(__ldg(&nd->x), fi32[k], -fK[k]);
+            ex[k] = crossing(k, __ldg(nd));
           }
         }
       }

@@ -47,3 +47,20 @@ def test_walk_bitwise(birp, oracle, layout, nodes, samples, length, segments):
                 ref = oracle.render64(oc, o_cam(oracle, cam), threads=THREADS).astype(np.float32)
                 assert np.array_equal(img, ref), (pos, fov, march, np.abs(img - ref).max())
     g.close()
+
+
+# Rays tilted against an axis by less and less, down to 1e-13: the walk's crossing index of a plane has 1 / (d dt) up
+# to 1e14 in it, and each of its estimates ends somewhere on the way.
+@pytest.mark.parametrize("tilt", [1e-4, 1e-6, 1e-8, 1e-9, 1e-10, 1e-11, 1e-13])
+@pytest.mark.parametrize("nodes,samples", [(17, 321), (33, 2000)])
+def test_walk_nearly_parallel(birp, oracle, tilt, nodes, samples):
+    axes, v, g = cube(birp, nodes, 1, nodes)
+    oc = oracle.Cube64(*axes, v.astype(np.float64), 0)
+    for fov in (1e-3, 1e3 * tilt):
+        for march in (birp.PREFIX, birp.CLIP):
+            cam = birp.camera((-7.5, tilt, -2 * tilt), (6.0, 0, 0), fov, fov, 9, 7, n_samples=samples, ray_length=17.0,
+                              trilinear=False, march=march)
+            img = birp.render(g, cam)
+            ref = oracle.render64(oc, o_cam(oracle, cam), threads=THREADS).astype(np.float32)
+            assert np.array_equal(img, ref), (fov, march, np.abs(img - ref).max())
+    g.close()
