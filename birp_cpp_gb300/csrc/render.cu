@@ -620,7 +620,8 @@ __device__ __noinline__ double cmem_value64(const CmemDev& m, bool need, double 
     const double angle = acos(role == 0   ? ct
                               : role == 1 ? ct * m.d_cos_tn + st * m.d_sin_tn * sp
                                           : ct * m.d_cos_ts - st * m.d_sin_ts * sp);
-    const double theta = x != 0 ? of(angle, 0) : 0.0, hh = theta / 2;
+    // (every lane takes part in every shuffle: x differs between the groups)
+    const double theta0 = of(angle, 0), theta = x != 0 ? theta0 : 0.0, hh = theta / 2;
     const double ex1 = exp(role == 0 ? -m.d_B * (hh * hh * hh * hh) : -theta);
     const double fb = sqrt(1 / bb) + m.d_a5 * (2 * st * ct) * (1 - of(ex1, 1));
     const double pw = pow(role == 0   ? r / 10
