@@ -29,6 +29,7 @@
 
 #include "birp_internal.h"
 #include "cell_index.h"
+#include "point_index.h"
 
 namespace birp {
 namespace {
@@ -2329,8 +2330,10 @@ __device__ __noinline__ float cube_point64(const CubeDev* Cp, float px, float py
 __global__ void cube_sample_kernel(const CubeDev* __restrict__ cube, int trilinear, const float* __restrict__ xyz,
                                    int n, float* __restrict__ out) {
   const CubeDev& C = *cube;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)n; t += gridDim.x * (size_t)blockDim.x) {
-    const float p[3] = {xyz[3 * t], xyz[3 * t + 1], xyz[3 * t + 2]};
+  const PointIndex step = points_step(gridDim.x, blockDim.x);
+  for (PointIndex t = points_first(blockIdx.x, blockDim.x, threadIdx.x); t < n; t += step) {
+    const float* const q = xyz + point_coords(t);
+    const float p[3] = {q[0], q[1], q[2]};
     bool in = true;
     int k[3];
     FF f[3];  // local coordinates (records) or fractions (node values)
@@ -2403,9 +2406,11 @@ __global__ void cmem_sample_kernel(const CmemDev* __restrict__ cmem, const float
                                    float* __restrict__ out) {
   const CmemFast fast = cmem_fast(*cmem);
   const float edge = cmem_edge(fast, 1e-6f);
-  for (int w = blockIdx.x * blockDim.x + (threadIdx.x & ~31); w < n; w += gridDim.x * blockDim.x) {  // whole warps
-    const int t = min(w + (int)(threadIdx.x & 31), n - 1);
-    const float x = xyz[3 * t], y = xyz[3 * t + 1], z = xyz[3 * t + 2];
+  const PointIndex step = points_step(gridDim.x, blockDim.x);
+  for (PointIndex w = points_first(blockIdx.x, blockDim.x, threadIdx.x & ~31); w < n; w += step) {  // whole warps
+    const PointIndex t = min(w + (PointIndex)(threadIdx.x & 31), (PointIndex)n - 1);
+    const float* const p = xyz + point_coords(t);
+    const float x = p[0], y = p[1], z = p[2];
     const bool far = !(fabsf(x) + fabsf(y) + fabsf(z) < 1e15f);  // or not a number
     float v = 0.f;
     bool open = false;
@@ -2739,8 +2744,8 @@ cudaError_t launch_cube_pairs(const float* padded, int nx, int ny, int nz, const
 cudaError_t launch_cube_sample(const CubeDev* cube, int trilinear, const float* xyz, int n, float* out,
                                cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  int blocks = std::min((n + 255) / 256, 4096);
-  cube_sample_kernel<<<blocks, 256, 0, s>>>(cube, trilinear, xyz, n, out);
+  const int blocks = point_blocks(n);
+  cube_sample_kernel<<<blocks, kPointThreads, 0, s>>>(cube, trilinear, xyz, n, out);
   return cudaGetLastError();
 }
 
@@ -2752,8 +2757,8 @@ cudaError_t launch_cmem_table(const CmemDev* cmem, float4* table, cudaStream_t s
 
 cudaError_t launch_cmem_sample(const CmemDev* cmem, const float* xyz, int n, float* out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  int blocks = std::min((n + 255) / 256, 4096);
-  cmem_sample_kernel<<<blocks, 256, 0, s>>>(cmem, xyz, n, out);
+  const int blocks = point_blocks(n);
+  cmem_sample_kernel<<<blocks, kPointThreads, 0, s>>>(cmem, xyz, n, out);
   return cudaGetLastError();
 }
 
