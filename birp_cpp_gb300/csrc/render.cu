@@ -1938,7 +1938,9 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         const int k = k0 + (lane >> 2) * 16 + warp * 4 + (lane & 3);
         const bool need = k < n;
         if (!__any_sync(0xffffffffu, need)) continue;
-        const int p = open.list[need ? k : k0], t = p / kOpen, i = open.at[p];
+        // (a lane without a place of its own computes on the first place's ray, but not from
+        // open.at, whose entry that place's own lane replaces by its value below)
+        const int p = open.list[need ? k : k0], t = p / kOpen, i = need ? open.at[p] : 0;
         const int tw = t >> 5, tr = (t & 31) >> SEGL2;
         const double* ta = sm.A[((tw & (WGX - 1)) << WBXL2) + (tr & (WBX - 1))];
         const double* tb = sm.B[(tw >> WGXL2) * WBY + (tr >> WBXL2)];
