@@ -901,7 +901,9 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
     }
     bool neg;
     FF val = {0.f, 0.f};
-    bool open = !(size < 1e37f);  // NaN, infinite or near-overflow corners
+    // NaN, infinite or near-overflow corners, and ones so small that the low
+    // parts fall under FP32's smallest step (the bounds below do not cover that)
+    bool open = !(size < 1e37f) || (size < 1e-20f && size > 0.f && !(mx < 0.f));
     if (!open) {
       if (mx < 0.f) {
         neg = true;  // every interpolation of negative corners is
