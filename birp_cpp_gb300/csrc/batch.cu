@@ -134,7 +134,7 @@ birp_status batch_create(int max_requests, int64_t max_pixels, birp_batch** out)
   return ok();
 }
 
-birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* const* direct_outs) {
+birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* const* direct_outs, bool waits) {
   if (birp_status s = check_init()) return s;
   if (!b || n < 0 || (n > 0 && !reqs)) return fail(BIRP_ERR_INVALID, "bad argument");
   if (n > b->max_req) return fail(BIRP_ERR_INVALID, "%d requests exceed the batch limit %d", n, b->max_req);
@@ -185,6 +185,7 @@ birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* 
     prefault_outputs(direct_outs, cnt.data(), n);
   }
   cudaError_t e;
+  for (int i = 0; i < n && !waits; ++i) note_async_use(reqs[i].cube);
   if ((e = cudaEventRecord(b->e_start, b->stream)) != cudaSuccess ||
       (e = cudaGraphLaunch(b->exec, b->stream)) != cudaSuccess ||
       (e = cudaEventRecord(b->e_kernel, b->stream)) != cudaSuccess ||
@@ -232,13 +233,14 @@ birp_status birp_batch_render(birp_batch* b, const birp_request* reqs, int n, fl
   if (n > 0 && !outs) return fail(BIRP_ERR_INVALID, "outs is NULL");
   bool direct = host_direct_writes() && n > 0;
   for (int i = 0; i < n && direct; ++i) direct = outs[i] != nullptr;
-  if (direct) {
-    // the kernel writes each image straight into the caller's buffer
-    if (birp_status s = batch_submit(b, reqs, n, outs)) return s;
-    return batch_wait(b);
+  // direct: the kernel writes each image straight into the caller's buffer
+  birp_status s = batch_submit(b, reqs, n, direct ? outs : nullptr, true);
+  if (s == BIRP_OK) s = batch_wait(b);
+  if (s != BIRP_OK) {
+    for (int i = 0; i < n && reqs; ++i) note_async_use(reqs[i].cube);  // perhaps launched, not waited for
+    return s;
   }
-  if (birp_status s = batch_submit(b, reqs, n)) return s;
-  if (birp_status s = batch_wait(b)) return s;
+  if (direct) return s;
   std::vector<const float*> src(n);
   std::vector<size_t> cnt(n);
   for (int i = 0; i < n; ++i) {

@@ -43,6 +43,7 @@ int request_class(const birp_request& r);
 birp_status batch_create(int max_requests, int64_t max_pixels, birp_batch** out);
 // direct_outs: when given, request i's image is written by the kernel into
 // direct_outs[i] (host memory the device can write) and nothing is copied back
-birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* const* direct_outs = nullptr);
+birp_status batch_submit(birp_batch* b, const birp_request* reqs, int n, float* const* direct_outs = nullptr,
+                         bool waits = false);
 birp_status batch_wait(birp_batch* b);
 }  // namespace birp

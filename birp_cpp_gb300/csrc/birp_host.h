@@ -32,6 +32,8 @@ struct birp_cube {
   size_t device_bytes = 0;
   cudaStream_t alloc_stream = nullptr;  // non-null: stream-ordered (pool) allocations
   size_t vals_bytes = 0, grid_bytes = 0, pairs_bytes = 0;  // of d_vals, d_grid and d_pairs (block_alloc)
+  int device = -1;                      // the device that holds it
+  mutable bool async_use = false;       // note_async_use (accessed atomically)
 };
 
 struct birp_cmem {
@@ -92,18 +94,25 @@ birp_status upload_cube(birp_cube& cube, const float* values, cudaStream_t strea
 // estimate of the device bytes a cube of these dims will hold
 size_t cube_device_bytes(const birp_cube& cube);
 // Device memory of cubes outside a server: blocks of at least 8 MB that a cube
-// gives back are kept, up to 1 GiB in all, for the next cube that needs nearly
-// as much (mapping and unmapping a 440 MB block takes 0.14 + 0.25 ms, a third
-// of a load). A block is kept only once the device is idle with respect to it,
-// so any stream may take it; the oldest go first when the bound is passed, all
-// go when an allocation fails and at birp_shutdown. Any thread.
+// gives back are kept, up to 1 GiB in all (block_cache.h), for the next cube
+// that needs nearly as much (mapping and unmapping a 440 MB block takes 0.14 +
+// 0.25 ms, a third of a load). A block is kept only once nothing on the device
+// uses it, so any stream may take it; the oldest go first when the bound is
+// passed, all go when an allocation fails and at birp_shutdown. Any thread.
+void blocks_open(int device);  // the device whose blocks are kept (birp_init)
+void blocks_close();           // frees them and keeps no more
 // *bytes: wanted, then what the block holds
 cudaError_t block_alloc(void** p, size_t* bytes);
-// device_idle: nothing on the device uses the block any more
-void block_free(void* p, size_t bytes, bool device_idle);
+// device: the one that holds it; device_idle: nothing there uses the block any more
+void block_free(void* p, size_t bytes, int device, bool device_idle);
 // cudaMalloc that gives the kept blocks back and tries again when memory is out
 cudaError_t device_alloc(void** p, size_t bytes);
 void block_release_all();
+// Notes that a call has put work on the cube into a stream and returned without
+// waiting for it (destroy_cube_device).
+inline void note_async_use(const birp_cube* c) {
+  if (c) __atomic_store_n(&c->async_use, true, __ATOMIC_RELEASE);
+}
 // whether any of the n values is below zero (a NaN is not)
 bool any_negative(const float* v, size_t n);
 void destroy_cube_device(birp_cube& cube);

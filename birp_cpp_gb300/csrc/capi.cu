@@ -368,6 +368,7 @@ birp_status birp_init(int device) {
   CK(cudaDeviceGetAttribute(&g_ctx.sms, cudaDevAttrMultiProcessorCount, device));
   CK(cudaDeviceGetAttribute(&g_ctx.pageable_access, cudaDevAttrPageableMemoryAccess, device));
   g_ctx.device = device;
+  blocks_open(device);
   return ok();
 }
 
@@ -376,7 +377,7 @@ void birp_shutdown(void) {
   if (g_ctx.device < 0) return;
   cudaSetDevice(g_ctx.device);
   cudaStreamSynchronize(g_ctx.stream);
-  block_release_all();
+  blocks_close();
   if (g_ctx.scratch) cudaFree(g_ctx.scratch);
   if (g_ctx.flush) cudaFree(g_ctx.flush);
   if (g_ctx.stats) cudaFree(g_ctx.stats);
@@ -438,7 +439,6 @@ birp_status birp_cube_create_layout(const double* xs, int nx, const double* ys, 
 
 birp_status birp_cube_destroy(birp_cube* cube) {
   if (!cube) return ok();
-  if (g_ctx.device >= 0) cudaStreamSynchronize(g_ctx.stream);
   destroy_cube_device(*cube);
   delete cube;
   return ok();
@@ -648,6 +648,7 @@ birp_status birp_render_device(const birp_cube* cube, const birp_cmem* cmem, con
   if (!out_device) return fail(BIRP_ERR_INVALID, "out_device is NULL");
   RequestDev r;
   if (birp_status s = build_request(cube, cmem, *cam, out_device, r)) return s;
+  if (stream) note_async_use(cube);
   CK(launch_render_plain(r, g_ctx.stats, pick_stream(stream)));
   return ok();
 }
@@ -661,18 +662,24 @@ birp_status birp_render(const birp_cube* cube, const birp_cmem* cmem, const birp
   const size_t npx = (size_t)cam->nx * cam->ny;
   cudaStream_t st = pick_stream(stream);
   RequestDev r;
+  cudaError_t e;
   if (host_direct_writes()) {
     // the kernel writes every pixel of the caller's image itself
     if (birp_status s = build_request(cube, cmem, *cam, out_host, r)) return s;
     prefault_outputs(&out_host, &npx, 1);
-    CK(launch_render_plain(r, g_ctx.stats, st));
+    e = launch_render_plain(r, g_ctx.stats, st);
   } else {
     if (birp_status s = ensure_scratch(npx)) return s;
     if (birp_status s = build_request(cube, cmem, *cam, g_ctx.scratch, r)) return s;
-    CK(launch_render_plain(r, g_ctx.stats, st));
-    CK(cudaMemcpyAsync(out_host, g_ctx.scratch, npx * sizeof(float), cudaMemcpyDeviceToHost, st));
+    e = launch_render_plain(r, g_ctx.stats, st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(out_host, g_ctx.scratch, npx * sizeof(float), cudaMemcpyDeviceToHost, st);
   }
-  CK(cudaStreamSynchronize(st));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    note_async_use(cube);  // not waited for
+    return fail(BIRP_ERR_CUDA, "render: %s", cudaGetErrorString(e));
+  }
   return ok();
 }
 

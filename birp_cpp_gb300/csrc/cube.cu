@@ -5,10 +5,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "birp_host.h"
+#include "block_cache.h"
 
 namespace birp {
 
@@ -100,22 +100,12 @@ birp_status ensure_xyz_scratch(size_t floats) {
 }
 
 namespace {
-struct Block {
-  void* p;
-  size_t bytes;
-};
-std::mutex g_blocks_mu;
-std::vector<Block> g_blocks;  // kept blocks, oldest first
-size_t g_blocks_bytes = 0;
-constexpr size_t kKeepMin = (size_t)8 << 20, kKeepMax = (size_t)1 << 30;
+BlockCache g_blocks([](void* p) { cudaFree(p); });
 }  // namespace
 
-void block_release_all() {
-  std::lock_guard<std::mutex> lk(g_blocks_mu);
-  for (const Block& b : g_blocks) cudaFree(b.p);
-  g_blocks.clear();
-  g_blocks_bytes = 0;
-}
+void blocks_open(int device) { g_blocks.open(device); }
+void blocks_close() { g_blocks.close(); }
+void block_release_all() { g_blocks.release_all(); }
 
 cudaError_t device_alloc(void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
@@ -128,39 +118,11 @@ cudaError_t device_alloc(void** p, size_t bytes) {
 }
 
 cudaError_t block_alloc(void** p, size_t* bytes) {
-  if (*bytes >= kKeepMin) {
-    std::lock_guard<std::mutex> lk(g_blocks_mu);
-    size_t best = g_blocks.size();
-    for (size_t i = 0; i < g_blocks.size(); ++i)  // the smallest that fits, at most an eighth larger
-      if (g_blocks[i].bytes >= *bytes && g_blocks[i].bytes <= *bytes + *bytes / 8 &&
-          (best == g_blocks.size() || g_blocks[i].bytes < g_blocks[best].bytes))
-        best = i;
-    if (best < g_blocks.size()) {
-      *p = g_blocks[best].p;
-      *bytes = g_blocks[best].bytes;
-      g_blocks_bytes -= g_blocks[best].bytes;
-      g_blocks.erase(g_blocks.begin() + (long)best);
-      return cudaSuccess;
-    }
-  }
-  return device_alloc(p, *bytes);
+  *p = g_blocks.take(g_ctx.device, bytes);
+  return *p ? cudaSuccess : device_alloc(p, *bytes);
 }
 
-void block_free(void* p, size_t bytes, bool device_idle) {
-  if (!p) return;
-  if (bytes < kKeepMin || bytes > kKeepMax || !device_idle || g_ctx.device < 0) {
-    cudaFree(p);
-    return;
-  }
-  std::lock_guard<std::mutex> lk(g_blocks_mu);
-  while (!g_blocks.empty() && g_blocks_bytes + bytes > kKeepMax) {
-    cudaFree(g_blocks.front().p);
-    g_blocks_bytes -= g_blocks.front().bytes;
-    g_blocks.erase(g_blocks.begin());
-  }
-  g_blocks.push_back({p, bytes});
-  g_blocks_bytes += bytes;
-}
+void block_free(void* p, size_t bytes, int device, bool device_idle) { g_blocks.give(p, bytes, device, device_idle); }
 
 void destroy_cube_device(birp_cube& c) {
   if (c.alloc_stream) {
@@ -169,11 +131,17 @@ void destroy_cube_device(birp_cube& c) {
                     (void*)c.d_grid, (void*)c.d_pairs, (void*)c.d_walk4, (void*)c.d_nodes_ff, (void*)c.d_negflag})
       if (p) cudaFreeAsync(p, c.alloc_stream);
   } else {
-    // a freed block waits for the device, and so does one that is kept
-    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
-    block_free(c.d_vals, c.vals_bytes, idle);
-    block_free(c.d_grid, c.grid_bytes, idle);
-    block_free(c.d_pairs, c.pairs_bytes, idle);
+    // A block is kept once nothing on the device uses it: the library's own
+    // stream is waited for, every other call that read the cube has waited for
+    // its work itself, and a cube read by one that did not (async_use) is freed,
+    // which waits for the device that holds it. (A wait for the whole device
+    // would be for the calling thread's current one, and is refused, breaking
+    // the capture, while any thread captures a stream.)
+    bool idle = g_ctx.device >= 0 && cudaStreamSynchronize(g_ctx.stream) == cudaSuccess;
+    idle = idle && !__atomic_load_n(&c.async_use, __ATOMIC_ACQUIRE);
+    block_free(c.d_vals, c.vals_bytes, c.device, idle);
+    block_free(c.d_grid, c.grid_bytes, c.device, idle);
+    block_free(c.d_pairs, c.pairs_bytes, c.device, idle);
     for (void* p : {(void*)c.d_c64, (void*)c.d_lut, (void*)c.d_desc, (void*)c.d_cells, (void*)c.d_walk4,
                     (void*)c.d_nodes_ff, (void*)c.d_negflag})
       if (p) cudaFree(p);
@@ -234,6 +202,7 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   const bool find_neg = direct && c.has_neg < 0;
   if (c.has_neg < 0) c.has_neg = !direct && any_negative(values, nodes) ? 1 : 0;
   c.alloc_stream = stream_alloc ? st : nullptr;
+  c.device = g_ctx.device;
 
   CubeDev& d = c.h_desc;
   std::memset(&d, 0, sizeof d);
@@ -453,7 +422,7 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
   CKU(cudaStreamSynchronize(st));
   if (!compact && !c.alloc_stream) {
     c.d_grid = nullptr;
-    block_free(scalar, c.grid_bytes, true);  // the stream that used it is done
+    block_free(scalar, c.grid_bytes, c.device, true);  // the stream that used it is done
   }
   return BIRP_OK;
 }

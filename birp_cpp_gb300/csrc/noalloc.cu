@@ -120,6 +120,7 @@ extern "C" birp_status birp_batch_render_noalloc(const birp_request* reqs, int n
   bd.reqs = reinterpret_cast<const RequestDev*>(scratch + kOffReqs);
   bd.counter = reinterpret_cast<unsigned int*>(scratch + kOffCounter);
   bd.stats = nullptr;
+  for (int i = 0; i < n && stream; ++i) note_async_use(reqs[i].cube);
   // the queue head must start at zero; the table is overwritten whole
   if ((e = cudaMemsetAsync(scratch + kOffCounter, 0, sizeof(unsigned int), st)) != cudaSuccess ||
       (e = cudaMemcpyAsync(scratch, g_stage, kOffReqs + (size_t)n * sizeof(RequestDev), cudaMemcpyHostToDevice,
