@@ -94,6 +94,7 @@ def lib():
             "birp_version": ([], I),
             "birp_init": ([I], I),
             "birp_shutdown": ([], None),
+            "birp_trim": ([], None),
             "birp_last_error": ([], C.c_char_p),
             "birp_cube_create": ([P, I, P, I, P, I, P, P], I),
             "birp_cube_create_layout": ([P, I, P, I, P, I, P, I, P], I),
@@ -155,6 +156,11 @@ def init(device: int = 0) -> None:
 
 def shutdown() -> None:
     lib().birp_shutdown()
+
+
+def trim() -> None:
+    """Gives back the device memory kept from destroyed cubes (birp_trim)."""
+    lib().birp_trim()
 
 
 def camera(pos, aim, fov_w, fov_h, nx, ny, n_samples=200, ray_length=44.0, trilinear=True, march=PREFIX,

@@ -98,7 +98,8 @@ size_t cube_device_bytes(const birp_cube& cube);
 // that needs nearly as much (mapping and unmapping a 440 MB block takes 0.14 +
 // 0.25 ms, a third of a load). A block is kept only once nothing on the device
 // uses it, so any stream may take it; the oldest go first when the bound is
-// passed, all go when an allocation fails and at birp_shutdown. Any thread.
+// passed, all go when an allocation of the library fails, at birp_trim and at
+// birp_shutdown. Any thread.
 void blocks_open(int device);  // the device whose blocks are kept (birp_init)
 void blocks_close();           // frees them and keeps no more
 // *bytes: wanted, then what the block holds

@@ -372,6 +372,8 @@ birp_status birp_init(int device) {
   return ok();
 }
 
+void birp_trim(void) { block_release_all(); }
+
 void birp_shutdown(void) {
   std::lock_guard<std::mutex> lk(g_ctx.mu);
   if (g_ctx.device < 0) return;
@@ -691,7 +693,7 @@ birp_status birp_time_render_device(const birp_cube* cube, const birp_cmem* cmem
   if (birp_status s = build_request(cube, cmem, *cam, out_device, r)) return s;
   cudaStream_t st = g_ctx.stream;
   const size_t flush_bytes = (size_t)512 << 20;  // larger than the 126 MB L2
-  if (flush_l2 && !g_ctx.flush) CK(cudaMalloc(&g_ctx.flush, flush_bytes));
+  if (flush_l2 && !g_ctx.flush) CK(device_alloc(&g_ctx.flush, flush_bytes));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -748,7 +750,7 @@ birp_status birp_flush_l2(void) {
   if (birp_status s = check_init()) return s;
   std::lock_guard<std::mutex> lk(g_ctx.mu);
   const size_t flush_bytes = (size_t)512 << 20;
-  if (!g_ctx.flush) CK(cudaMalloc(&g_ctx.flush, flush_bytes));
+  if (!g_ctx.flush) CK(device_alloc(&g_ctx.flush, flush_bytes));
   static unsigned char v = 0;
   CK(cudaMemsetAsync(g_ctx.flush, ++v, flush_bytes, g_ctx.stream));
   CK(cudaStreamSynchronize(g_ctx.stream));
@@ -767,8 +769,8 @@ birp_status birp_measure_peaks(double* fp32_tflops, double* l2_read_gbs, size_t*
   // each SM the same slice in every repetition, which L1 would otherwise
   // serve), each launch reading about 2 GB, best of 3 launches per size
   const size_t max_bytes = (size_t)64 << 20;
-  CK(cudaMalloc(&sink, sizeof(float)));
-  CK(cudaMalloc(&buf, max_bytes));
+  CK(device_alloc((void**)&sink, sizeof(float)));
+  CK(device_alloc((void**)&buf, max_bytes));
   CK(cudaMemsetAsync(buf, 0, max_bytes, st));
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));

@@ -46,6 +46,12 @@ int birp_version(void);
 birp_status birp_init(int device);
 /* Frees the library's device state. Handles must be destroyed first. */
 void birp_shutdown(void);
+/* Gives back the device memory that destroyed cubes have left for the next
+ * ones: up to 1 GiB in blocks of 8 MB and more, which the library otherwise
+ * gives back by itself when an allocation of its own fails and at
+ * birp_shutdown. For programs whose other allocators need that memory. No
+ * reference counterpart. Any thread. */
+void birp_trim(void);
 /* Message of the last failing call on this thread ("" if none). */
 const char* birp_last_error(void);
 
