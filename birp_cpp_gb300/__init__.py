@@ -118,6 +118,7 @@ def lib():
             "birp_batch_last_ms": ([P, P, P], I),
             "birp_batch_upload_bytes": ([P, P], I),
             "birp_debug_bounds": ([P, I], I),
+            "birp_debug_bounds_codes": ([P], I),
             "birp_server_default_config": ([P], None),
             "birp_server_create": ([P, P], I),
             "birp_server_destroy": ([P], I),
@@ -452,3 +453,9 @@ def debug_bounds(reset: bool = True) -> int:
     check(lib().birp_debug_bounds(C.byref(st), int(reset)))
     return st.value
 
+
+def debug_bounds_codes() -> int:
+    """Codes of the accesses the bounds-checking build has checked (bit c: code c; birp_debug_bounds_codes)."""
+    codes = C.c_ulonglong()
+    check(lib().birp_debug_bounds_codes(C.byref(codes)))
+    return codes.value

@@ -203,8 +203,9 @@ cudaError_t launch_cube_fill(const float* src_xfast, int nx, int ny, int nz, flo
 cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, int* neg, cudaStream_t stream);
 cudaError_t launch_cube_negflags(const float* padded, int nx, int ny, int nz, uint8_t* flags, cudaStream_t stream);
 // bounds-checking build: the first out-of-range access (code << 48 | index),
-// 0 if none, optionally reset; other builds: always 0, returns false
-bool read_bounds_status(unsigned long long* status, bool reset);
+// 0 if none, and the codes of which an access was checked (bit c: code c),
+// optionally reset; other builds: always 0, returns false
+bool read_bounds_status(unsigned long long* status, unsigned long long* codes, bool reset);
 // iwx, iwy, iwz: the inverse widths of cells -1..n-1 (0 for the guard cells) as
 // float pairs (device)
 cudaError_t launch_cube_records(const float* padded, int nx, int ny, int nz, const float2* iwx, const float2* iwy,

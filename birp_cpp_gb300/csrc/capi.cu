@@ -718,8 +718,21 @@ birp_status birp_debug_bounds(unsigned long long* status, int reset) {
   if (birp_status s = check_init()) return s;
   if (!status) return fail(BIRP_ERR_INVALID, "NULL argument");
   CK(cudaDeviceSynchronize());
-  if (!read_bounds_status(status, reset != 0)) {
+  unsigned long long codes = 0;
+  if (!read_bounds_status(status, &codes, reset != 0)) {
     *status = 0;
+    return fail(BIRP_ERR_INVALID, "not a bounds-checking build (BIRP_DEBUG_BOUNDS)");
+  }
+  return ok();
+}
+
+birp_status birp_debug_bounds_codes(unsigned long long* codes) {
+  if (birp_status s = check_init()) return s;
+  if (!codes) return fail(BIRP_ERR_INVALID, "NULL argument");
+  CK(cudaDeviceSynchronize());
+  unsigned long long status = 0;
+  if (!read_bounds_status(&status, codes, false)) {
+    *codes = 0;
     return fail(BIRP_ERR_INVALID, "not a bounds-checking build (BIRP_DEBUG_BOUNDS)");
   }
   return ok();

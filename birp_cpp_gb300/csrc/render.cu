@@ -64,9 +64,14 @@ constexpr int kMagicBits = 0x4B400000;
 #ifdef BIRP_DEBUG_BOUNDS
 // Bounds-checking build: the first out-of-range table access of any kernel
 // (code << 48 | index); the caller then redirects the access to a valid
-// element, so a violation is reported, never a fault.
-__device__ unsigned long long g_bounds_status;
+// element, so a violation is reported, never a fault. Codes: 1 index tables,
+// 2 node values, 3 negative-value flags, 4 the box's planes, 5 walk tables,
+// 6 records, 7 node grids, 8 the nearest walk's planes and 9 values, 10 the
+// planes of signed_cell and 11 of nearest_run_exact, 12 the CMEM table; bit c
+// of g_bounds_codes: an access of code c was checked.
+__device__ unsigned long long g_bounds_status, g_bounds_codes;
 __device__ __forceinline__ bool bound_ok(long long i, long long n, unsigned long long code) {
+  if (!((*(volatile unsigned long long*)&g_bounds_codes >> code) & 1)) atomicOr(&g_bounds_codes, 1ull << code);
   if (i >= 0 && i < n) return true;
   atomicCAS(&g_bounds_status, 0ull, (code << 48) | ((unsigned long long)i & 0xffffffffffffull));
   return false;
@@ -574,6 +579,13 @@ __device__ __forceinline__ bool cmem_by_table(const CmemFast& m, float x, float 
   const float ryz2 = fmaxf(fmaf(y, y, z * z), 1e-30f), r2 = fmaf(x, x, ryz2);
   const float ir = rsqrt_fast(r2), r = r2 * ir, ct = x * ir, cp = y * rsqrt_fast(ryz2);
   const float4 e = __ldg(m.table + cmem_table_index(ct, cp));  // r_mp, r_mp, r_bs, r_bs: min, max
+#ifdef BIRP_DEBUG_BOUNDS
+  // (the index is masked to the table for any argument: here, that none is needed for a direction)
+  if (ryz2 > off_axis) {
+    bound_ok((int)(__float_as_uint(fmaf(ct, kCtScale, kMagic + (0.5f * kCmemCt - 1.f))) - kMagicBits), kCmemCt, 12);
+    bound_ok((int)(__float_as_uint(fmaf(cp, kCpScale, kMagic + (0.5f * kCmemCp - 1.f))) - kMagicBits), kCmemCp, 12);
+  }
+#endif
   const float h = fmaf(m.eps_rel, r, edge), up = r + h, lo = r - h;
   const bool known = ryz2 > off_axis && x * y != 0.f;
   const bool past = lo > e.y, in0 = up < e.x, in2 = known && past && up < e.z, in4 = past && lo > e.w;
@@ -819,6 +831,9 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
     const float mid = 0.5f * (float)(i0 + i1 - 1), m = (float)(i1 - i0);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
+#ifdef BIRP_DEBUG_BOUNDS
+      if (!bound_ok(k[r], C.ax[r].n - 1, 10)) k[r] = 0;
+#endif
       const float2 c0 = __ldg(C.nodes_ff[r] + k[r]), c1 = __ldg(C.nodes_ff[r] + k[r] + 1);
       for (int last = 0; last < 2; ++last) {
         const FF x = ff_add(bs[r], ff_mul(st[r], {(float)(last ? i1 - 1 : i0), 0.f}));
@@ -876,6 +891,9 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
       const FF x = ff_add(bs[r], ff_mul(st[r], {(float)i, 0.f}));
       // whether the oracle's position lies below node j
       auto below = [&](int j) {
+#ifdef BIRP_DEBUG_BOUNDS
+        if (!bound_ok(j, A.n, 10)) j = 0;
+#endif
         const float2 c = __ldg(C.nodes_ff[r] + j);
         const float diff = (x.hi - c.x) + (x.lo - c.y);
         if (fabsf(diff) > e[r]) return diff < 0.f;
@@ -886,6 +904,9 @@ __device__ __noinline__ LaneRun signed_cell(const RequestDev* Rp, const double* 
       };
       while (k[r] > 0 && below(k[r])) --k[r];
       while (k[r] < A.n - 2 && !below(k[r] + 1)) ++k[r];
+#ifdef BIRP_DEBUG_BOUNDS
+      if (!bound_ok(k[r], A.n - 1, 10)) k[r] = 0;
+#endif
       const float2 c0 = __ldg(C.nodes_ff[r] + k[r]), c1 = __ldg(C.nodes_ff[r] + k[r] + 1);
       const FF iw = ff_recip(ff_add({c1.x, c1.y}, {-c0.x, -c0.y}));
       f[r] = ff_mul(ff_add(x, {-c0.x, -c0.y}), iw);
@@ -977,6 +998,9 @@ __device__ __noinline__ LaneRun nearest_run_exact(const RequestDev* Rp, const do
     const bool up = d[k] > 0.0;
     const int j = up ? c[k] + 1 : c[k];
     if (j < 0 || j >= C.ax[k].n) return never;  // beyond the box
+#ifdef BIRP_DEBUG_BOUNDS
+    if (!bound_ok(C.nodes_ff[k] + j - (C.nodes_ff[0] - 1), C.nodes_n, 11)) return never;
+#endif
     const float2 P = __ldg(C.nodes_ff[k] + j);
     const FF u = ff_add(ff_mul({P.x, P.y}, inv[k]), {-K[k].hi, -K[k].lo});
     if (!(u.hi <= (float)R.N + 1.5f)) return never;
@@ -1468,6 +1492,9 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         // infinite exit plane), which has no flag.
         if constexpr (SIGNED) {
           const unsigned fc = min((unsigned)fi, flags_end);
+#ifdef BIRP_DEBUG_BOUNDS
+          if (nxt > u && fmaxf(fmaxf(ex[0], ex[1]), ex[2]) != INFINITY) bound_ok(fi, C.neg_n, 3);
+#endif
           flagged = nxt > u && (all_exact || __ldg(C.negflag + fc) || fmaxf(fmaxf(ex[0], ex[1]), ex[2]) == INFINITY);
           if (!__any_sync(walkers, u < ub && !flagged)) break;
         }
@@ -1752,6 +1779,9 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         fK[k] = good ? K[k].hi : 3e38f;
         fil[k] = good ? inv[k].lo : 0.f;
         fKl[k] = good ? K[k].lo : 0.f;
+#ifdef BIRP_DEBUG_BOUNDS
+        if (!bound_ok(np[k] - (C.nodes_ff[0] - 1), C.nodes_n, 8)) np[k] = C.nodes_ff[0];
+#endif
         ni[k] = (int)(np[k] - nbase);
         ex[k] = w64[k] == 0.0 ? INFINITY : crossing(k, __ldg(np[k]));
       }
@@ -2688,16 +2718,20 @@ cudaError_t launch_render_batch(const BatchDev& b, int grid, cudaStream_t s, int
   return cudaGetLastError();
 }
 
-bool read_bounds_status(unsigned long long* status, bool reset) {
+bool read_bounds_status(unsigned long long* status, unsigned long long* codes, bool reset) {
 #ifdef BIRP_DEBUG_BOUNDS
-  if (cudaMemcpyFromSymbol(status, g_bounds_status, sizeof *status) != cudaSuccess) return false;
+  if (cudaMemcpyFromSymbol(status, g_bounds_status, sizeof *status) != cudaSuccess ||
+      cudaMemcpyFromSymbol(codes, g_bounds_codes, sizeof *codes) != cudaSuccess)
+    return false;
   if (reset) {
     const unsigned long long zero = 0;
-    if (cudaMemcpyToSymbol(g_bounds_status, &zero, sizeof zero) != cudaSuccess) return false;
+    if (cudaMemcpyToSymbol(g_bounds_status, &zero, sizeof zero) != cudaSuccess ||
+        cudaMemcpyToSymbol(g_bounds_codes, &zero, sizeof zero) != cudaSuccess)
+      return false;
   }
   return true;
 #else
-  *status = 0;
+  *status = *codes = 0;
   (void)reset;
   return false;
 #endif

@@ -240,10 +240,15 @@ birp_status birp_batch_upload_bytes(const birp_batch* b, size_t* bytes);
  * every table access of the render kernels; the first out-of-range one is
  * recorded (code << 48 | index; codes: 1 index table, 2 node value, 3
  * negative-value flag, 4 box plane, 5 walk table, 6 cell record, 7 padded
- * grid, 8 node plane, 9 nearest value) and redirected to a valid element.
+ * grid, 8 node plane, 9 nearest value, 10 node plane of a cell next to a
+ * negative node, 11 node plane of a nearest run decided in FP64, 12 CMEM table)
+ * and redirected to a valid element.
  * Gives that status (0: none) and resets it when `reset`; in other builds
  * *status = 0 and BIRP_ERR_INVALID. No counterpart in the reference. */
 birp_status birp_debug_bounds(unsigned long long* status, int reset);
+/* The codes of which accesses have been checked since the last reset (bit c:
+ * code c), for tests that each of them is reached. */
+birp_status birp_debug_bounds_codes(unsigned long long* codes);
 
 /* ---------------------------------------------------------------- serving */
 
