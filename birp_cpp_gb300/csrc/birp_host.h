@@ -55,9 +55,16 @@ struct Context {
   size_t xyz_floats = 0;
   void* flush = nullptr;         // L2 flush buffer (timing)
   int pageable_access = 0;       // kernels may write pageable host memory
+  // Pinned host memory that small inputs go through (birp_cube_sample,
+  // birp_cmem_sample, cube values): copied by the host and read by the kernel
+  // there, without a device copy and without the translation of pages the
+  // device has not used lately (2-4 us an array). nullptr: none.
+  float* stage = nullptr;
+  std::mutex stage_mu;           // held while a call uses it
   std::mutex mu;
 };
 extern Context g_ctx;
+constexpr size_t kStageFloats = 32768;  // 128 KB (the figures beside each use)
 
 // True when render outputs in host memory are written by the kernels
 // directly (the device reads and writes pageable host memory coherently,
