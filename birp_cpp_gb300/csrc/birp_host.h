@@ -27,7 +27,7 @@ struct birp_cube {
   float2* d_pairs = nullptr;    // pairs layout: padded {value, z-slope} per node
   float4* d_walk4 = nullptr;    // compact and pairs layouts: walk tables with inverse widths
   float2* d_nodes_ff = nullptr; // node coordinates as float pairs, 3 axes concatenated
-  int has_neg = -1;             // a value below zero (-1: not yet known)
+  int has_neg = -1;             // values below zero (birp::NegKind; -1: not yet known)
   uint8_t* d_negflag = nullptr; // its negative-value flags (CubeDev::negflag)
   size_t device_bytes = 0;
   cudaStream_t alloc_stream = nullptr;  // non-null: stream-ordered (pool) allocations

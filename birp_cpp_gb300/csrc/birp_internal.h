@@ -116,6 +116,10 @@ struct CmemDev {
 };
 constexpr int kCmemCt = 256, kCmemCp = 64;
 
+// Whether a cube holds values below zero (it then carries flags), and how many
+// (upload_cube).
+enum NegKind : int { NEG_NONE = 0, NEG_FEW = 1, NEG_MANY = 2 };
+
 enum SpaceKind : int { SPACE_CUBE = 0, SPACE_CMEM = 1 };
 // Device layouts of a cube (the values of BIRP_CUBE_*).
 enum CubeLayout : int { CUBE_RECORDS = 0, CUBE_COMPACT = 1, CUBE_PAIRS = 2 };
@@ -145,7 +149,7 @@ struct RequestDev {
   int tiles_x;       // tiles along x for this request's tile shape
   int tiles;         // total tiles
   int layout;        // cube: CUBE_RECORDS, CUBE_COMPACT or CUBE_PAIRS
-  int has_neg;       // cube: 1 when it holds a value below zero (it carries flags)
+  int has_neg;       // cube: whether it holds values below zero (NegKind)
   const CubeDev* cube;   // device pointer (kind == SPACE_CUBE)
   const CmemDev* cmem;   // device pointer (kind == SPACE_CMEM)
   float* out;            // ny*nx floats, row 0 = top
@@ -201,7 +205,9 @@ cudaError_t launch_cube_fill(const float* src_xfast, int nx, int ny, int nz, flo
 // the interior of the padded grid; *neg (device, nullptr: not wanted) becomes 1
 // if one is below zero
 cudaError_t launch_cube_pad_copy(const float* src, int nx, int ny, int nz, float* dst, int* neg, cudaStream_t stream);
-cudaError_t launch_cube_negflags(const float* padded, int nx, int ny, int nz, uint8_t* flags, cudaStream_t stream);
+// the flags of the nodes next to a value below zero, and the number of such values (device)
+cudaError_t launch_cube_negflags(const float* padded, int nx, int ny, int nz, uint8_t* flags, unsigned* count,
+                                 cudaStream_t stream);
 // bounds-checking build: the first out-of-range access (code << 48 | index),
 // 0 if none, and the codes of which an access was checked (bit c: code c),
 // optionally reset; other builds: always 0, returns false

@@ -249,7 +249,7 @@ birp_status build_request(const birp_cube* cube, const birp_cmem* cmem, const bi
   if (cube) {
     r.cube = cube->d_desc;
     r.layout = cube->layout;
-    r.has_neg = cube->has_neg > 0 ? 1 : 0;
+    r.has_neg = std::max(cube->has_neg, 0);
   } else {
     r.cmem = cmem->d_desc;
   }

@@ -287,9 +287,10 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
       }
   }
   const size_t iw_off = (total * sizeof(float) + 7) / 8 * 8, neg_off = iw_off + iw.size() * sizeof(float2);
-  CKU(big_alloc(&scalar, &c.grid_bytes, neg_off + (find_neg ? sizeof(int) : 0), c.alloc_stream));
+  CKU(big_alloc(&scalar, &c.grid_bytes, neg_off + 2 * sizeof(int), c.alloc_stream));
   float2* const d_iw = reinterpret_cast<float2*>(reinterpret_cast<char*>(scalar) + iw_off);
   int* const d_neg = find_neg ? reinterpret_cast<int*>(reinterpret_cast<char*>(scalar) + neg_off) : nullptr;
+  unsigned* const d_count = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(scalar) + neg_off) + 1;
   c.d_grid = scalar;
   if (nodes_layout) {
     CKU(dev_alloc(&c.d_walk4, walk.size() * sizeof(float4), c.alloc_stream));
@@ -338,7 +339,20 @@ birp_status upload_cube(birp_cube& c, const float* values, cudaStream_t st, bool
       c.device_bytes += nodes;
     }
   }
-  if (c.has_neg) CKU(launch_cube_negflags(scalar, nx, ny, nz, c.d_negflag, st));
+  if (c.has_neg) {
+    // Many: more than 1 % of the values (trilinear rays are gone over in windows,
+    // SignedRay). us a view of 144x144 pixels, 200 samples (576x336, 880; 32x24,
+    // 20000), whole rays against windows, random signs: 1e-5 of the values 40 (158;
+    // 21) and 51 (184; 34), 0.1 % 182 (1270; 2534) and 195 (1267; 2483), 1 % 482 (5155;
+    // 5335) and 475 (4867; 5117), 10 % 810 (7573; 9514) and 527 (7471; 7468), 50 % 287
+    // (382; 6508) and 113 (397; 1581), 95 % 65 (38; 744) and 31 (38; 14); a smooth field
+    // of both signs 269 (1238; 4910) and 231 (1296; 2986).
+    unsigned count = 0;
+    CKU(launch_cube_negflags(scalar, nx, ny, nz, c.d_negflag, d_count, st));
+    CKU(cudaMemcpyAsync(&count, d_count, sizeof count, cudaMemcpyDeviceToHost, st));
+    CKU(cudaStreamSynchronize(st));
+    c.has_neg = count > nodes / 100 ? NEG_MANY : NEG_FEW;
+  }
   if (!iw.empty()) CKU(cudaMemcpyAsync(d_iw, iw.data(), iw.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
   // (the host vectors below stay alive until the synchronize at the end)
   std::vector<double> all;
