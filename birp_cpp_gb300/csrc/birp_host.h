@@ -16,6 +16,7 @@ struct birp_cube {
   int uniform[3] = {0, 0, 0};
   double inv_h[3] = {0, 0, 0};  // uniform axes: 1 / spacing
   double min_gap[3] = {0, 0, 0};
+  double cells_per_length[3] = {0, 0, 0};  // mean along each axis
   birp::CubeDev h_desc{};       // host copy of the device descriptor
   birp::CubeDev* d_desc = nullptr;
   float4* d_vals = nullptr;     // cell records (birp_internal.h)

@@ -150,6 +150,7 @@ struct RequestDev {
   int tiles;         // total tiles
   int layout;        // cube: CUBE_RECORDS, CUBE_COMPACT or CUBE_PAIRS
   int has_neg;       // cube: whether it holds values below zero (NegKind)
+  int coarse;        // cube: its samples are several cells apart (build_request)
   const CubeDev* cube;   // device pointer (kind == SPACE_CUBE)
   const CmemDev* cmem;   // device pointer (kind == SPACE_CMEM)
   float* out;            // ny*nx floats, row 0 = top

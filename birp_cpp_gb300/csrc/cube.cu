@@ -30,6 +30,7 @@ birp_status analyze_axis(const double* c, int n, char name, birp_cube& cube, int
   cube.uniform[k] = uniform ? 1 : 0;
   cube.inv_h[k] = 1.0 / h;
   cube.min_gap[k] = min_gap;
+  cube.cells_per_length[k] = 1.0 / h;
   const double span = c[n - 1] - c[0];
   if (span / min_gap > (double)kMaxLutBins)
     return fail(BIRP_ERR_INVALID, "axis %c: span / smallest cell = %.0f exceeds %d", name, span / min_gap,

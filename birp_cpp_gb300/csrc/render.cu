@@ -1166,7 +1166,10 @@ enum Axes { AXES_NONE = 0, AXES_DDA = 2, AXES_DDA_COMPACT = 3, AXES_DDA_PAIRS = 
 // the cells next to a negative node in float-float (signed_cell) and finds the
 // run's ends there; the nearest march of such a cube finds them by the cells'
 // own values.
-template <int KIND, int INTERP, int AXES, bool SIGNED = false>
+// COARSE: the trilinear march of a request whose samples are several cells apart
+// (RequestDev::coarse): a cell without a sample is neither loaded nor summed,
+// which costs a divergent branch a cell.
+template <int KIND, int INTERP, int AXES, bool SIGNED = false, bool COARSE = false>
 __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty, TileSmem& sm,
                                             KernelStats* stats) {
   const int SEGL2 = R.seg_log2;
@@ -1506,6 +1509,10 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
         all_exact = fmaf(e_pos, C.neg_inv_gap, 2e-6f * (float)C.neg_nmax + 1e-6f) >= 1.f;
       }
       while (SIGNED || u < ub) {
+        // the first sample past the cell; not behind u, where a plane passed
+        // before sample u is still to be stepped (such a cell holds no sample)
+        if constexpr (COARSE) nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
+        if (!COARSE || nxt > u) {
         float4 lo, hi;  // {c0, c3, c1, c5}, {c2, c6, c4, c7}
         if constexpr (COMPACT) {
           // the cell's trilinear coefficients from its 8 corners, in local
@@ -1550,9 +1557,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
               : "=f"(lo.x), "=f"(lo.y), "=f"(lo.z), "=f"(lo.w), "=f"(hi.x), "=f"(hi.y), "=f"(hi.z), "=f"(hi.w)
               : "l"(q));
         }
-        // the first sample past the cell; not behind u, where a plane passed
-        // before sample u is still to be stepped (such a cell holds no sample)
-        nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
+        if constexpr (!COARSE) nxt = fmaxf(fminf(ceilf(fminf(fminf(ex[0], ex[1]), ex[2])), ub), u);
         // a cube holding negative values: the samples of a cell next to a
         // negative node are looked at by signed_cell; an unflagged cell's are
         // all good, as its FP32 cell is within one of the exact one (unless
@@ -1630,6 +1635,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
           acc.add_product(m, any ? mean : 0.f);
           ncell += any ? 1.f : 0.f;
           u = SIGNED && flagged ? u : nxt;
+        }
         }
         // step each axis whose exit index has been reached, once: a second
         // plane passed before the next sample is stepped in the next
@@ -2111,11 +2117,11 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
 }
 
 // One request, one CTA per tile; the request travels as a kernel parameter.
-template <int KIND, int INTERP, int AXES, bool SIGNED = false>
+template <int KIND, int INTERP, int AXES, bool SIGNED = false, bool COARSE = false>
 __global__ void __launch_bounds__(kThreads) render_plain_kernel(const __grid_constant__ RequestDev req,
                                                                 KernelStats* stats) {
   __shared__ TileSmem sm;
-  render_tile<KIND, INTERP, AXES, SIGNED>(req, blockIdx.x, blockIdx.y, sm, stats);
+  render_tile<KIND, INTERP, AXES, SIGNED, COARSE>(req, blockIdx.x, blockIdx.y, sm, stats);
 }
 
 // The nearest and compact-layout trilinear marches alone, compiled for the
@@ -2141,6 +2147,13 @@ __device__ __forceinline__ void render_tile_nearest(const RequestDev& R, int tx,
   }
 }
 
+// A trilinear tile of a cube without negative values.
+template <int AXES>
+__device__ __forceinline__ void render_tile_tri(const RequestDev& R, int tx, int ty, TileSmem& sm, KernelStats* st) {
+  if (!R.coarse) render_tile<SPACE_CUBE, TRILINEAR, AXES>(R, tx, ty, sm, st);
+  else render_tile<SPACE_CUBE, TRILINEAR, AXES, false, true>(R, tx, ty, sm, st);
+}
+
 // Dispatch over the request's variant.
 __device__ void render_tile_any(const RequestDev& R, int tx, int ty, TileSmem& sm, KernelStats* st) {
   if (R.kind == SPACE_CMEM) {
@@ -2150,9 +2163,9 @@ __device__ void render_tile_any(const RequestDev& R, int tx, int ty, TileSmem& s
     else if (R.layout == CUBE_PAIRS) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, true>(R, tx, ty, sm, st);
     else render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA, true>(R, tx, ty, sm, st);
   } else if (R.interp) {
-    if (R.layout == CUBE_COMPACT) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT>(R, tx, ty, sm, st);
-    else if (R.layout == CUBE_PAIRS) render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS>(R, tx, ty, sm, st);
-    else render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA>(R, tx, ty, sm, st);
+    if (R.layout == CUBE_COMPACT) render_tile_tri<AXES_DDA_COMPACT>(R, tx, ty, sm, st);
+    else if (R.layout == CUBE_PAIRS) render_tile_tri<AXES_DDA_PAIRS>(R, tx, ty, sm, st);
+    else render_tile_tri<AXES_DDA>(R, tx, ty, sm, st);
   } else {
     render_tile_nearest(R, tx, ty, sm, st);
   }
@@ -2195,11 +2208,11 @@ __global__ void __launch_bounds__(kThreads, CLS == BATCH_ANY          ? 1
     const int t = item - __ldg(B.first + lo);
     const int tx = t % R.tiles_x, ty = t / R.tiles_x;
     if constexpr (CLS == BATCH_CUBE_TRI) {
-      render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA>(R, tx, ty, sm, B.stats);
+      render_tile_tri<AXES_DDA>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_TRI_COMPACT) {
-      render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT>(R, tx, ty, sm, B.stats);
+      render_tile_tri<AXES_DDA_COMPACT>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_TRI_PAIRS) {
-      render_tile<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS>(R, tx, ty, sm, B.stats);
+      render_tile_tri<AXES_DDA_PAIRS>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CMEM) {
       render_tile<SPACE_CMEM, TRILINEAR, AXES_NONE>(R, tx, ty, sm, B.stats);
     } else if constexpr (CLS == BATCH_CUBE_NEAREST) {
@@ -2763,6 +2776,12 @@ cudaError_t launch_render_plain(const RequestDev& h, KernelStats* stats, cudaStr
     render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.has_neg)
     render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA, true><<<grid, kThreads, 0, s>>>(h, stats);
+  else if (h.interp && h.coarse && h.layout == CUBE_COMPACT)
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_COMPACT, false, true><<<grid, kThreads, 0, s>>>(h, stats);
+  else if (h.interp && h.coarse && h.layout == CUBE_PAIRS)
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA_PAIRS, false, true><<<grid, kThreads, 0, s>>>(h, stats);
+  else if (h.interp && h.coarse)
+    render_plain_kernel<SPACE_CUBE, TRILINEAR, AXES_DDA, false, true><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.layout == CUBE_COMPACT)
     render_plain_cube_kernel<TRILINEAR, AXES_DDA_COMPACT, BIRP_COMPACT_MINB><<<grid, kThreads, 0, s>>>(h, stats);
   else if (h.interp && h.layout == CUBE_PAIRS)
