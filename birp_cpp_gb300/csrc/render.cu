@@ -555,10 +555,8 @@ __device__ __forceinline__ CmemEval cmem_value32(const CmemDev& m, float x, floa
 // alone. Returns false (the full computation decides) next to a surface, next
 // to the Earth-Sun line (ryz2 <= off_axis), and for x = 0 or y = 0, whose
 // angles the reference sets to 0.
-// Sheath value: exp(-B (theta/2)^4) multiplies it by 1 - 6 B at most, and B
-// is the field in tesla (~1e-8), so theta to 7e-5 is enough (the table's
-// r_bs bounds say so: unknown where B > 1e-5): acos by Abramowitz and Stegun
-// 4.4.45, |error| <= 6.8e-5.
+// The angle of a sheath sample: acos by Abramowitz and Stegun 4.4.46, |error|
+// <= 2e-8 (5e-7 with its FP32 evaluation, as cmem_theta's).
 // Bound by instruction issue (~62 a sample, from ~205 through the radii; 2 %
 // of the samples still take those). 12 orbit views (2.67e9 samples) 14.1 ->
 // 5.2 ms, a 144x144 view of 200 samples 149 -> 67 us, with the FP64 samples
@@ -577,7 +575,7 @@ __device__ __forceinline__ float cmem_edge(const CmemFast& m, float perr) { retu
 __device__ __forceinline__ bool cmem_by_table(const CmemFast& m, float x, float y, float z, float edge, float off_axis,
                                               float& v) {
   const float ryz2 = fmaxf(fmaf(y, y, z * z), 1e-30f), r2 = fmaf(x, x, ryz2);
-  const float ir = rsqrt_fast(r2), r = r2 * ir, ct = x * ir, cp = y * rsqrt_fast(ryz2);
+  const float ir = rsqrt_fast(r2), iyz = rsqrt_fast(ryz2), r = r2 * ir, ct = x * ir, cp = y * iyz;
   const float4 e = __ldg(m.table + cmem_table_index(ct, cp));  // r_mp, r_mp, r_bs, r_bs: min, max
 #ifdef BIRP_DEBUG_BOUNDS
   // (the index is masked to the table for any argument: here, that none is needed for a direction)
@@ -591,12 +589,17 @@ __device__ __forceinline__ bool cmem_by_table(const CmemFast& m, float x, float 
   const bool past = lo > e.y, in0 = up < e.x, in2 = known && past && up < e.z, in4 = past && lo > e.w;
   v = in0 ? 0.f : m.A2k * (ir * ir * ir);
   if (in2) {
-    const float c = fabsf(ct);
-    float p = fmaf(c, -0.0187293f, 0.0742610f);
-    p = fmaf(p, c, -0.2121144f);
-    p = fmaf(p, c, 1.5707288f);
-    const float t = sqrt_fast(fmaxf(1.f - c, 0.f)) * p, hh = 0.5f * (ct < 0.f ? 3.14159274f - t : t);
-    const float h4 = (hh * hh) * (hh * hh), st2 = ryz2 * ir * ir;
+    // theta = acos(ct): sqrt(1 - |ct|) = sin theta / sqrt(1 + |ct|), exact towards the axis
+    const float c = fabsf(ct), st = ryz2 * iyz * ir;
+    float p = fmaf(c, -0.0012624911f, 0.0066700901f);
+    p = fmaf(p, c, -0.0170881256f);
+    p = fmaf(p, c, 0.0308918810f);
+    p = fmaf(p, c, -0.0501743046f);
+    p = fmaf(p, c, 0.0889789874f);
+    p = fmaf(p, c, -0.2145988016f);
+    p = fmaf(p, c, 1.5707963050f);
+    const float t = st * rsqrt_fast(1.f + c) * p, hh = 0.5f * (ct < 0.f ? 3.14159274f - t : t);
+    const float h4 = (hh * hh) * (hh * hh), st2 = st * st;
     // log2(r / 10) as half the log2 of (r / 10)^2
     v = m.A1 * ex2_fast(fmaf(m.nB, h4, fmaf(m.n_beta, st2, m.n_alpha) * (0.5f * __log2f(r2 * 0.01f))));
   }
@@ -2637,8 +2640,6 @@ __global__ void cmem_table_kernel(const CmemDev* __restrict__ cmem, float4* __re
   };
   mp = widen(mp);
   bs = widen(bs);
-  // a sheath value needs theta to full precision where B is not small
-  if (!(m.B <= 1e-5f)) bs.lo = -INFINITY;
   table[t] = make_float4(mp.lo, mp.hi, bs.lo, bs.hi);
 }
 
