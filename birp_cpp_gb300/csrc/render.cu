@@ -606,63 +606,98 @@ __device__ __forceinline__ bool cmem_by_table(const CmemFast& m, float x, float 
   return in2 || (known && (in0 || in4));
 }
 
-// The same in FP64 for the lanes of a warp that need it, whole warps only: the
-// FP64 oracle's formulas (oracle cmem64_sample), with the direction's cosines
-// and sines taken from the position instead of through acos (equal to ~1e-16;
-// the reference's theta = 0 at x = 0 and phi = 0 at y = 0 kept). An FP64
+// The value in FP64 at radius r, the radii known: the oracle's branch chain.
+__device__ __forceinline__ double cmem_shell64(const CmemDev& m, double r, double r_mp, double r_bs, double sheath) {
+  const double half = (double)(0.05f / 2);
+  const double d10 = r / 10, outer = m.d_A2 * (1 / (d10 * d10 * d10));
+  if (r < r_mp - half) return 0.0;
+  if (r >= r_mp - half && r <= r_mp + half) return (r - (r_mp - half)) / (r_mp + half) * sheath;  // lerp(0, sheath, t)
+  if (r > r_mp + half && r < r_bs - half) return sheath;
+  if (r >= r_bs - half && r <= r_bs + half) return sheath + (r - (r_bs - half)) / (r_bs + half) * (outer - sheath);
+  return outer;
+}
+
+// The same in FP64 for one sample: the FP64 oracle's formulas (oracle
+// cmem64_sample), with the direction's cosines and sines taken from the position
+// instead of through acos (equal to ~1e-16; the reference's theta = 0 at x = 0
+// and phi = 0 at y = 0 kept).
+struct CmemDir64 {
+  double r, ct, st, cp, sp, bb;  // bb = 2 / (1 + cos theta) without its cancellation towards the tail
+};
+__device__ __forceinline__ CmemDir64 cmem_dir64(double x, double y, double z) {
+  const double ryz2 = y * y + z * z, r = sqrt(x * x + ryz2), ryz = sqrt(ryz2);
+  return {r,
+          x != 0 ? x / r : 1.0,
+          x != 0 ? ryz / r : 0.0,
+          y != 0 ? y / ryz : 1.0,
+          y != 0 ? fabs(z) / ryz : 0.0,
+          x == 0  ? 1.0
+          : x > 0 ? 2 * r / (r + x)
+                  : 2 * r * (r - x) / ryz2};
+}
+__device__ __noinline__ double cmem_lane64(const CmemDev& m, double x, double y, double z) {
+  const CmemDir64 d = cmem_dir64(x, y, z);
+  const double theta = x != 0 ? acos(d.ct) : 0.0, hh = theta / 2;
+  const double phi_n = acos(d.ct * m.d_cos_tn + d.st * m.d_sin_tn * d.sp);
+  const double phi_s = acos(d.ct * m.d_cos_ts - d.st * m.d_sin_ts * d.sp);
+  const double fb = sqrt(1 / d.bb) + m.d_a5 * (2 * d.st * d.ct) * (1 - exp(-theta));
+  const double f = pow(fb, m.d_p1 * (m.d_bc0 + m.d_bc1 * d.cp + m.d_bc3 * (d.sp * d.sp)));
+  const double q = m.d_p2 * m.d_charlie * exp(m.d_p3 * m.d_dn * pow(phi_n, m.d_a21)) +
+                   m.d_p2 * m.d_charlie * exp(m.d_p3 * m.d_ds * pow(phi_s, m.d_a21));
+  const double ry = m.d_bs * pow(d.bb, m.d_ay), rz = m.d_bs * pow(d.bb, m.d_az);
+  const double a1 = rz * d.cp, a2 = ry * d.sp;
+  const double sheath = m.d_A1 * exp(-m.d_B * (hh * hh * hh * hh)) * pow(d.r / 10, -m.d_alpha - m.d_beta * (d.st * d.st));
+  return cmem_shell64(m, d.r, m.d_p0 * m.d_r0 * f + q, (ry * rz) / sqrt(a1 * a1 + a2 * a2), sheath);
+}
+
+// The same for the lanes of a warp that need it, whole warps only. An FP64
 // instruction costs a warp the same for 1 lane as for 32, so 8 lanes share a
 // sample: its acos, exp, pow and exp calls each run once, every lane of the
 // group on another argument (4 calls in a row instead of 28; 4 samples at a
-// time). Returns each needing lane its own value.
+// time). Where more than kCmemLanes lanes need it (a model whose radii are not
+// numbers leaves every sample open) each computes its own: 144x144 pixels of 200
+// samples of such a model 24.3 ms shared, 7.9 so. Returns each needing lane its
+// own value.
+constexpr int kCmemLanes = 12;
 __device__ __noinline__ double cmem_value64(const CmemDev& m, bool need, double px, double py, double pz) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, role = lane & 7, base = lane & 24;
-  const double half = (double)(0.05f / 2);
   double mine = 0.0;
-  for (unsigned todo = __ballot_sync(kAll, need); todo != 0;) {
+  unsigned todo = __ballot_sync(kAll, need);
+  if (__popc(todo) > kCmemLanes) return need ? cmem_lane64(m, px, py, pz) : 0.0;
+  while (todo != 0) {
     // this group's sample: the todo's (lane / 8)-th lane (its first, unused, when there are fewer)
     unsigned t = todo;
     for (int j = 0; j < base; j += 8) t &= t - 1;
     const int owner = t ? __ffs(t) - 1 : -1, src = t ? owner : __ffs(todo) - 1;
     const double x = __shfl_sync(kAll, px, src), y = __shfl_sync(kAll, py, src), z = __shfl_sync(kAll, pz, src);
     auto of = [&](double v, int r) { return __shfl_sync(kAll, v, base + r); };  // lane r of the group
-    const double ryz2 = y * y + z * z, r = sqrt(x * x + ryz2), ryz = sqrt(ryz2);
-    const double ct = x != 0 ? x / r : 1.0, st = x != 0 ? ryz / r : 0.0;
-    const double cp = y != 0 ? y / ryz : 1.0, sp = y != 0 ? fabs(z) / ryz : 0.0;
-    // 2 / (1 + cos theta) without its cancellation towards the tail
-    const double bb = x == 0 ? 1.0 : x > 0 ? 2 * r / (r + x) : 2 * r * (r - x) / ryz2;
+    const CmemDir64 d = cmem_dir64(x, y, z);
     // angles: theta, and phi_n, phi_s to the cusp axes (cos(phi - pi/2) = sin
     // phi, cos(phi - 3 pi/2) = -sin phi)
-    const double angle = acos(role == 0   ? ct
-                              : role == 1 ? ct * m.d_cos_tn + st * m.d_sin_tn * sp
-                                          : ct * m.d_cos_ts - st * m.d_sin_ts * sp);
+    const double angle = acos(role == 0   ? d.ct
+                              : role == 1 ? d.ct * m.d_cos_tn + d.st * m.d_sin_tn * d.sp
+                                          : d.ct * m.d_cos_ts - d.st * m.d_sin_ts * d.sp);
     // (every lane takes part in every shuffle: x differs between the groups)
     const double theta0 = of(angle, 0), theta = x != 0 ? theta0 : 0.0, hh = theta / 2;
     const double ex1 = exp(role == 0 ? -m.d_B * (hh * hh * hh * hh) : -theta);
-    const double fb = sqrt(1 / bb) + m.d_a5 * (2 * st * ct) * (1 - of(ex1, 1));
-    const double pw = pow(role == 0   ? r / 10
+    const double fb = sqrt(1 / d.bb) + m.d_a5 * (2 * d.st * d.ct) * (1 - of(ex1, 1));
+    const double pw = pow(role == 0   ? d.r / 10
                           : role <= 2 ? angle
                           : role == 3 ? fb
-                                      : bb,
-                          role == 0   ? -m.d_alpha - m.d_beta * (st * st)
+                                      : d.bb,
+                          role == 0   ? -m.d_alpha - m.d_beta * (d.st * d.st)
                           : role <= 2 ? m.d_a21
-                          : role == 3 ? m.d_p1 * (m.d_bc0 + m.d_bc1 * cp + m.d_bc3 * (sp * sp))
+                          : role == 3 ? m.d_p1 * (m.d_bc0 + m.d_bc1 * d.cp + m.d_bc3 * (d.sp * d.sp))
                           : role == 4 ? m.d_ay
                                       : m.d_az);
     const double ex2 = exp((role == 1 ? m.d_p3 * m.d_dn : m.d_p3 * m.d_ds) * pw);
     const double q = m.d_p2 * m.d_charlie * of(ex2, 1) + m.d_p2 * m.d_charlie * of(ex2, 2);
     const double r_mp = m.d_p0 * m.d_r0 * of(pw, 3) + q;
     const double ry = m.d_bs * of(pw, 4), rz = m.d_bs * of(pw, 5);
-    const double a1 = rz * cp, a2 = ry * sp;
+    const double a1 = rz * d.cp, a2 = ry * d.sp;
     const double r_bs = (ry * rz) / sqrt(a1 * a1 + a2 * a2);
-    const double sheath = m.d_A1 * of(ex1, 0) * of(pw, 0);
-    const double d10 = r / 10, outer = m.d_A2 * (1 / (d10 * d10 * d10));
-    double v;
-    if (r < r_mp - half) v = 0.0;
-    else if (r >= r_mp - half && r <= r_mp + half) v = (r - (r_mp - half)) / (r_mp + half) * sheath;  // lerp(0, sheath, t)
-    else if (r > r_mp + half && r < r_bs - half) v = sheath;
-    else if (r >= r_bs - half && r <= r_bs + half) v = sheath + (r - (r_bs - half)) / (r_bs + half) * (outer - sheath);
-    else v = outer;
+    const double v = cmem_shell64(m, d.r, r_mp, r_bs, m.d_A1 * of(ex1, 0) * of(pw, 0));
     for (int j = 0; j < 32; j += 8) {
       const int o = __shfl_sync(kAll, owner, j);
       const double w = __shfl_sync(kAll, v, j);

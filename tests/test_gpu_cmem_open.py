@@ -60,3 +60,36 @@ def test_groups_of_a_warp(birp, oracle, kw):
     alone = np.array([model.sample(q[None])[0] for q in p], np.float32)
     assert np.array_equal(got, alone)
     model.close()
+
+
+@pytest.mark.parametrize("count", [1, 4, 5, 12, 13, 31, 32])
+def test_open_samples_in_a_warp(birp, oracle, count):
+    """Up to 12 open samples of a warp share its lanes, more take a lane each: the same values."""
+    om = oracle.Cmem64()
+    rng = np.random.default_rng(count)
+    p = np.full((32, 3), 3.0, np.float32)  # inside the magnetopause: decided without them
+    p[:, 0] = np.linspace(-3, 3, 32)
+    at = rng.permutation(32)[:count]
+    p[at] = edge_points(om, rng.integers(0, 3, count), count)
+    model = birp.Cmem()
+    got = model.sample(p)
+    assert np.array_equal(got, np.array([model.sample(q[None])[0] for q in p], np.float32))
+    ref = om.sample(p.astype(np.float64))
+    assert np.array_equal(got == 0, ref == 0)
+    assert np.max(np.abs(got - ref)[ref != 0] / ref[ref != 0]) <= TOL
+    model.close()
+
+
+def test_radii_that_are_not_numbers(birp, oracle):
+    """A model whose radii are NaN leaves every sample open: the oracle's outer values, in calls and in renders."""
+    kw = dict(density=-5.0)
+    om, model = oracle.Cmem64(oracle.cmem_args(**kw)), birp.Cmem(birp.cmem_params(**kw))
+    p = np.random.default_rng(2).uniform(-20, 20, (3000, 3)).astype(np.float32)
+    with np.errstate(all="ignore"):
+        ref = om.sample(p.astype(np.float64))
+        assert np.max(np.abs(model.sample(p) - ref) / ref) <= TOL
+        cam = birp.camera((5.9, 6.7, 17.7), (9, 0, 0), 40.0, 30.0, 19, 13, n_samples=120)
+        img = birp.render(model, cam)
+        want = oracle.render64(om, oracle.camera64(tuple(cam.pos), tuple(cam.aim), 40.0, 30.0, 19, 13, 120), threads=4)
+    assert np.max(np.abs(img - want) / want) <= TOL
+    model.close()
