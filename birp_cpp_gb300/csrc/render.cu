@@ -2410,7 +2410,10 @@ __global__ void cube_records_kernel(const float* __restrict__ v, int nx, int ny,
     float coefs = 0.f;
 #pragma unroll
     for (int k = 1; k < 8; ++k) coefs += fabsf(o[k]);
-    if (!(size == 0.f || (size > 1e-20f && size < 1e30f && coefs < 1e30f))) {
+    // (and cells wider than 1e10: a product of their inverse widths has no room for
+    // its low part)
+    auto wide = [](float iw) { return iw != 0.f && iw < 1e-10f; };
+    if (!(size == 0.f || (size > 1e-20f && size < 1e30f && coefs < 1e30f)) || wide(fx.x) || wide(fy.x) || wide(fz.x)) {
       const float f[8] = {v000, v001, v010, v011, v100, v101, v110, v111};
       const double i3[3] = {(double)fx.x + fx.y, (double)fy.x + fy.y, (double)fz.x + fz.y};
       cell_record64(f, i3, o);
