@@ -33,6 +33,10 @@ over all 512 requests.
              then p50/p99 at 70% of that saturated rate, with parity of
              served images
 
+The result is one JSON line on stdout of at most 2400 characters, with the
+single numbers of each block; `--details FILE` writes all of it (per-image
+errors, every rate and size).
+
 `--impl reference` times only the CPU implementation (bounded samples).
 `--workload c3|c4` runs one of the extra blocks alone (`--c4-layout`,
 `--c4-promote-layout`, `--c4-promote-gb`, `--c4-uploaders` vary the config-4
@@ -466,7 +470,7 @@ def run_c4(args, B, O):
     for rate in (float(r) for r in args.c4_rates.split(",")):
         r = phase(rate, args.c4_seconds)
         sweep.append(r)
-        print(json.dumps({"c4_rate": r}), file=sys.stderr, flush=True)
+        print("c4 rate:", json.dumps(r), file=sys.stderr, flush=True)
         sat = max(sat, r["served_images_s"])
         if r["served_images_s"] < 0.9 * rate:
             break
@@ -690,6 +694,8 @@ def main():
     ap.add_argument("--cpu-seconds", type=float, default=10.0)
     ap.add_argument("--serve-seconds", type=float, default=3.0)
     ap.add_argument("--parity-px", type=int, default=256, help="pixels checked per image against the FP64 oracle")
+    ap.add_argument("--details", help="file for everything measured (per-image errors, every rate and size), as JSON; "
+                                      "the line on stdout has the single numbers")
     ap.add_argument("--no-plain", action="store_true")
     ap.add_argument("--no-c3", action="store_true", help="skip the config-3 block of the default run")
     ap.add_argument("--no-c4", action="store_true", help="skip the config-4 block of the default run")
@@ -954,7 +960,51 @@ def main():
             "c3": c3, "c4": c4,
             "parity": parity,
         }
-        print(json.dumps(line))
+        print_result(line, args.details)
+
+
+# What the result line keeps of its larger blocks, and the longest it may get:
+# programs that read the end of a run's output keep 2 to 3 KB of it.
+BRIEF = {
+    "e2e_breakdown": ("kernel_ms", "host_ms"), "serving": ("achieved_images_s", "p50_ms", "p99_ms"),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac"), "roofline_issue": ("achieved", "peak", "unit", "frac"),
+    "cpu_baseline": ("value", "unit", "cores", "kind"), "c3": ("requests", "images_s", "batched_vs_plain", "parity"),
+    "c4": ("saturation_images_s", "at_70pct_of_saturation", "parity"),
+    "parity": ("images", "pixels_checked", "max_rel_err", "rms_rel_err", "images_within_tolerance", "tolerance"),
+}
+BRIEF_NESTED = ("max_rel_err", "images_within_tolerance", "served_images_s", "p50_ms", "p99_ms")
+WHOLE = ("config", "e2e", "clocks", "plain")
+MAX_LINE = 2400
+
+
+def result_line(full: dict) -> str:
+    """The result as one JSON line of at most MAX_LINE characters: every plain
+    value and the config, clocks, end-to-end and launch counts in full, of the
+    other blocks the numbers BRIEF names."""
+    def short(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+
+    line = {}
+    for k, v in full.items():
+        if not isinstance(v, (dict, list)):
+            line[k] = v if k in ("value", "ms_per_step") else short(v)
+        elif k in WHOLE:
+            line[k] = v
+        elif k in BRIEF:
+            line[k] = {a: {n: short(x[n]) for n in BRIEF_NESTED if n in x} if isinstance(x, dict) else short(x)
+                       for a, x in ((a, v[a]) for a in BRIEF[k] if a in v)}
+    for k in ("e2e_breakdown", "c4", "c3", "serving", "roofline_issue"):  # (not reached by the blocks as they are)
+        if len(json.dumps(line)) > MAX_LINE:
+            line.pop(k, None)
+    return json.dumps(line)
+
+
+def print_result(full: dict, details: str | None) -> None:
+    """The result line on stdout; everything measured in the file `details`."""
+    if details:
+        with open(details, "w") as f:
+            json.dump(full, f)
+    print(result_line(full), flush=True)
 
 
 def serve_latency(B, W, rate: float, seconds: float, seed: int = 13):
