@@ -40,8 +40,8 @@ errors, every rate and size).
 `--impl reference` times only the CPU implementation (bounded samples).
 `--workload c3|c4` runs one of the extra blocks alone (`--c4-layout`,
 `--c4-promote-layout`, `--c4-promote-gb`, `--c4-uploaders` vary the config-4
-server); `--profile-case trilinear|nearest|compact|pairs|cmem` runs a small
-fixed batch to profile one kernel class. Multi-GPU (torchrun): replicas, one per rank, barrier + max
+server); `--profile-case trilinear|nearest|compact|pairs|cmem|signed` runs a
+small fixed batch to profile one kernel class. Multi-GPU (torchrun): replicas, one per rank, barrier + max
 over ranks (the c3/c4 blocks run at N = 1 only).
 """
 from __future__ import annotations
@@ -557,8 +557,9 @@ def run_c4(args, B, O):
 def run_profile_case(args):
     """A small fixed batch for profiling one kernel class: the first
     --requests requests of the orbit sampler on the 256^3 stretched cube
-    (trilinear or nearest, records, pairs or compact layout) or on the
-    default CMEM model, launched --launches times."""
+    (trilinear or nearest, records, pairs or compact layout; signed: 1e-5 of
+    its nodes negative) or on the default CMEM model, launched --launches
+    times."""
     import birp_cpp_gb300 as B
     from birp_cpp_gb300 import build, synth
     build.build()
@@ -569,6 +570,8 @@ def run_profile_case(args):
         space = B.Cmem()
     else:
         xs, ys, zs, v = synth.cube_config1(seed=1)
+        if mode == "signed":
+            v = np.where(np.random.default_rng(5).random(v.shape) < 1e-5, -0.01 * v - 1e-4, v)
         layout = {"compact": B.CUBE_COMPACT, "pairs": B.CUBE_PAIRS}.get(mode, B.CUBE_RECORDS)
         space = B.Cube(xs, ys, zs, v.astype(np.float32), layout=layout)
     cams = [B.camera(p, a, synth.FOV_W, synth.FOV_H, nx, ny, n_samples=synth.n_samples(s),
@@ -702,7 +705,7 @@ def main():
     ap.add_argument("--workload", default="c2", choices=["c2", "c3", "c4"],
                     help="c2: the default run (headline on config 2, plus the c3 and c4 blocks); c3 / c4: that "
                          "block alone")
-    ap.add_argument("--profile-case", choices=["trilinear", "nearest", "compact", "pairs", "cmem"],
+    ap.add_argument("--profile-case", choices=["trilinear", "nearest", "compact", "pairs", "cmem", "signed"],
                     help="run a small fixed batch of one kernel class (for a profiler) and exit")
     ap.add_argument("--launches", type=int, default=4, help="launches of --profile-case")
     ap.add_argument("--c4-cubes", type=int, default=256)

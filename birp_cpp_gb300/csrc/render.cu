@@ -2185,11 +2185,19 @@ __device__ __forceinline__ void render_tile_nearest(const RequestDev& R, int tx,
   }
 }
 
-// A trilinear tile of a cube without negative values.
+// A trilinear tile of a cube without negative values. (The order of the two
+// marches is the compiler's order too: 64 orbit renders records 6.13 ms with the
+// common one first, 6.15 with the coarse one, compact 8.98 and 8.73, pairs 7.15
+// and 7.11.)
 template <int AXES>
 __device__ __forceinline__ void render_tile_tri(const RequestDev& R, int tx, int ty, TileSmem& sm, KernelStats* st) {
-  if (!R.coarse) render_tile<SPACE_CUBE, TRILINEAR, AXES>(R, tx, ty, sm, st);
-  else render_tile<SPACE_CUBE, TRILINEAR, AXES, false, true>(R, tx, ty, sm, st);
+  if constexpr (AXES == AXES_DDA) {
+    if (!R.coarse) render_tile<SPACE_CUBE, TRILINEAR, AXES>(R, tx, ty, sm, st);
+    else render_tile<SPACE_CUBE, TRILINEAR, AXES, false, true>(R, tx, ty, sm, st);
+  } else {
+    if (R.coarse) render_tile<SPACE_CUBE, TRILINEAR, AXES, false, true>(R, tx, ty, sm, st);
+    else render_tile<SPACE_CUBE, TRILINEAR, AXES>(R, tx, ty, sm, st);
+  }
 }
 
 // Dispatch over the request's variant.
