@@ -33,7 +33,9 @@ def nvcc() -> str:
 
 
 def _flags():
-    return ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
+    # (kernels stored as they are: above some size nvcc compresses them, and the
+    # first launch of a process then takes 11 ms instead of 1.5)
+    return ARCH + ["--no-compress", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
                    "-I", os.path.join(HERE, "..", "include")]
 
 
