@@ -232,7 +232,8 @@ CLASSES = {  # class: (macro, candidates of resident CTAs per SM, profile case)
     "compact": ("BIRP_COMPACT_MINB", [5, 6, 7, 8], "compact"),
     "pairs": ("BIRP_PAIRS_MINB", [6, 7, 8], "pairs"),
     "nearest": ("BIRP_NEAREST_MINB", [6, 7, 8], "nearest"),
-    "cmem": ("BIRP_CMEM_MINB", [5, 6, 7, 8, 9, 10, 12], "cmem"),
+    "cmem": ("BIRP_CMEM_MINB", [5, 6, 7, 8, 9, 10], "cmem"),
+    "signed": ("BIRP_SIGNED_MINB", [5, 6, 7, 8], "signed"),
 }
 
 
@@ -256,6 +257,8 @@ if mode == "cmem":
     space = B.Cmem()
 else:
     xs, ys, zs, v = synth.cube_config1(seed=1)
+    if mode == "signed":
+        v = np.where(np.random.default_rng(5).random(v.shape) < 1e-5, -0.01 * v - 1e-4, v)
     layout = {{"compact": B.CUBE_COMPACT, "pairs": B.CUBE_PAIRS}}.get(mode, B.CUBE_RECORDS)
     space = B.Cube(xs, ys, zs, v.astype(np.float32), layout=layout)
 cams = [B.camera(p, a, synth.FOV_W, synth.FOV_H, nx, ny, n_samples=synth.n_samples(s), trilinear=mode != "nearest")
@@ -301,8 +304,9 @@ def write_launch(occ, path):
     lines = ["// Resident CTAs per SM each persistent batch kernel class is compiled for",
              "// (__launch_bounds__ minimum; fewer allow more registers per thread). Written",
              "// by birp_cpp_gb300/autotune.py from the batch kernel's time on a fixed",
-             "// workload per class (64 orbit requests on the 256^3 stretched cube, 16 on the",
-             "// default CMEM model) with each candidate, on a GB300."]
+             "// workload per class (64 orbit requests on the 256^3 stretched cube, signed: 1e-5",
+             "// of its nodes negative; 16 on the default CMEM model) with each candidate, on a",
+             "// GB300."]
     for cls, (macro, _c, _case) in CLASSES.items():
         times = ", ".join(f"{k}: {t:.3f} ms" for k, t in sorted(occ[cls][1].items()))
         lines.append(f"#define {macro}_TUNED {occ[cls][0]}  // {times}")

@@ -7,11 +7,11 @@
 // by dt * 637810000 / (4/pi) / 1e4 (src/Camera.cpp:201).
 //
 // GB300 design:
-//  * One CTA renders a pixel tile; each warp marches a small 2D block of rays
-//    in lockstep in t, so the 32 lanes of a gather hit neighbouring cells.
-//    A ray may be split over S = 2^k lanes that take interleaved samples
-//    (lane s takes i = a + s, a + s + S, ...), merged by a compensated
-//    shuffle tree; this keeps gathers coalesced while shortening long rays.
+//  * One CTA renders a pixel tile; each warp marches a small 2D block of rays,
+//    so the 32 lanes of a gather hit neighbouring cells. A ray may be split
+//    over S = 2^k lanes, merged by a compensated shuffle tree, which shortens
+//    long rays: a cube's walks take contiguous parts of its samples, CMEM's
+//    lanes interleaved ones (lane s: i = a + s, a + s + S, ...).
 //  * FP32 marching with per-lane Kahan sums. FP64 (1/58 of FP32 rate on GB300)
 //    is used only where a decision must agree with the FP64 oracle exactly:
 //    the per-ray in-box sample range (certified by an FP32 error bound, redone
@@ -54,9 +54,7 @@ constexpr int kThreads = 128;
 #define BIRP_CMEM_MINB BIRP_CMEM_MINB_TUNED  // CMEM
 #endif
 #ifndef BIRP_SIGNED_MINB
-// trilinear cubes holding negative values (any layout; 12 views, mean of 12 sets,
-// at 5, 6, 7 and 8 CTAs per SM: 1.59, 1.56, 1.61, 1.64 ms)
-#define BIRP_SIGNED_MINB 6
+#define BIRP_SIGNED_MINB BIRP_SIGNED_MINB_TUNED  // trilinear cubes holding negative values (any layout)
 #endif
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;
@@ -2164,8 +2162,7 @@ __global__ void __launch_bounds__(kThreads) render_plain_kernel(const __grid_con
 
 // The nearest and compact-layout trilinear marches alone, compiled for the
 // resident CTAs per SM of their batch classes (16 orbit renders, one call
-// each: nearest 4.82 -> 4.58 ms, compact 4.62 -> 4.48 ms; the records and
-// pairs marches no faster).
+// each: nearest 3.19 -> 3.16 ms, compact 3.54 -> 3.53 ms).
 template <int INTERP, int AXES, int MINB, bool SIGNED = false>
 __global__ void __launch_bounds__(kThreads, MINB) render_plain_cube_kernel(const __grid_constant__ RequestDev req,
                                                                            KernelStats* stats) {
