@@ -711,7 +711,12 @@ __device__ __noinline__ double cmem_value64(const CmemDev& m, bool need, double 
 // takes the pipe as long for one lane as for 32, and a call inside the march
 // costs it registers. Each thread has kOpen places; a march that fills them
 // pauses for the tile to evaluate and goes on.
-constexpr int kOpen = 4;
+// On long rays a pass is at most kOpenSpan samples a lane: threads fill their
+// places at different samples, and those that pause early would wait for the
+// others to go all the way, pass after pass (64x48 rays of 400000 samples 60 ms
+// without the limit, 28 with it, 35 with the FP64 call inside the march; 12 rays
+// of 4 million 305, 180 and 380).
+constexpr int kOpen = 4, kOpenSpan = 4096;
 struct CmemOpen {
   int n;                                  // filled places of the tile
   unsigned short list[kThreads * kOpen];  // the places, packed
@@ -2077,6 +2082,7 @@ __device__ __forceinline__ void render_tile(const RequestDev& R, int tx, int ty,
       // (the loop's one exit is its condition: with a break in the branch the
       // warp's lanes do not come together again after it)
       float stop = end;
+      if (iters > kOpenSpan) stop = fminf(end, fi + (float)kOpenSpan * fS);
 #pragma unroll 1
       while (fi < stop) {
         const float x = fmaf(fi, st[0], bs[0]) + fmaf(fi, st_lo[0], bs_lo[0]);
